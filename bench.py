@@ -249,7 +249,7 @@ def run_gpu(args):
     csr = centrality._primal_csr(ns)
     wsp = centrality._workspace(ns, csr, 0, K, speed, max(s))
     sp = centrality.prepare_source_sampling(ns, None, None, None, None)
-    proc_t = torch.from_numpy(sp.process).to(dev)
+    proc_t = torch.from_numpy(centrality.spatial_order(ns, sp.process)).to(dev)
     wt_t = torch.from_numpy(sp.src_wt).to(dev)
     el_t = torch.from_numpy(sp.eligible).to(dev)
     q = centrality._make_query(d, b, s, speed, float(centrality.TIE_EPSILON), True, True, False, proc_t, wt_t,

@@ -58,7 +58,8 @@ class Call:
 
 def _plan_tensors(ns, source_indices, dev):
     sp = centrality.prepare_source_sampling(ns, None, None, None, source_indices)
-    keep = [torch.from_numpy(np.ascontiguousarray(x)).to(dev) for x in (sp.process, sp.src_wt, sp.eligible)]
+    process = sp.process if ns.is_dual else centrality.spatial_order(ns, sp.process)
+    keep = [torch.from_numpy(np.ascontiguousarray(x)).to(dev) for x in (process, sp.src_wt, sp.eligible)]
     return sp, keep
 
 

@@ -242,6 +242,55 @@ def _primal_csr(ns) -> device.PrimalCSR:
     return c
 
 
+def _hilbert_rank(ns) -> np.ndarray:
+    """Each node index's place along a Hilbert curve over the nodes' coordinates (once per graph)."""
+    rank = ns._cache.get("hilbert_rank")
+    if rank is not None:
+        return rank
+    nb = ns.node_bound()
+    x, y = (np.nan_to_num(np.array(c.view()[:nb], np.float64)) for c in (ns._x, ns._y))
+    bits = 16
+    span = max(float(np.ptp(x)), float(np.ptp(y)), 1e-9) if nb else 1.0
+    scale = ((1 << bits) - 1) / span
+    px = ((x - x.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
+    py = ((y - y.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
+    key = np.zeros(nb, np.int64)
+    for b in range(bits - 1, -1, -1):
+        rx, ry = (px >> b) & 1, (py >> b) & 1
+        key = (key << 2) | ((3 * rx) ^ ry)
+        # the quadrant's curve is the base curve mirrored and transposed
+        flip = (ry == 0) & (rx == 1)
+        mask = (1 << b) - 1
+        px, py = px & mask, py & mask
+        px, py = np.where(flip, mask - px, px), np.where(flip, mask - py, py)
+        swap = ry == 0
+        px, py = np.where(swap, py, px), np.where(swap, px, py)
+    rank = np.empty(nb, np.int64)
+    rank[np.argsort(key, kind="stable")] = np.arange(nb)
+    ns._cache["hilbert_rank"] = rank
+    return rank
+
+
+TILE_CALL = 8192  # no smaller call has a tile of 32 sources for every resident block
+
+
+def spatial_order(ns, process: np.ndarray) -> np.ndarray:
+    """The sources of a large call reordered so that consecutive ones lie near one another: the tile
+    kernel takes 32 consecutive sources per block, and their searches share what their reaches have in
+    common (on the 202,500-node lattice at 5 km, rows of 32 nodes instead of compact groups cost it
+    2.3x).  Smaller calls keep their order."""
+    process = np.ascontiguousarray(process, np.int32)
+    if len(process) < TILE_CALL:
+        return process
+    at = _hilbert_rank(ns)[process]
+    placed = np.full(ns.node_bound(), -1, np.int32)
+    placed[at] = process
+    out = placed[placed >= 0]
+    if len(out) != len(process):  # a source listed more than once
+        out = process[np.argsort(at, kind="stable")]
+    return out
+
+
 def drop_device_state(ns, keep_workspace: bool = True) -> None:
     """Forgets the device-resident CSR (and optionally the workspaces) of a graph."""
     for k in list(ns._cache):
@@ -409,7 +458,7 @@ def shortest_rows(ns, sp: SourcePlan, process: np.ndarray, dists, bets, secs, sp
     K = len(dists)
     csr = _primal_csr(ns)
     dev = csr.device
-    proc_t = torch.from_numpy(np.ascontiguousarray(process, np.int32)).to(dev)
+    proc_t = torch.from_numpy(spatial_order(ns, process)).to(dev)
     wt_t = torch.from_numpy(sp.src_wt).to(dev)
     el_t = torch.from_numpy(sp.eligible).to(dev)
     g = csr.struct(speed)
@@ -475,7 +524,7 @@ def betweenness_od_shortest(ns, od_matrix: OdMatrix, distances=None, betas=None,
     ptr_t = torch.from_numpy(ptr.astype(np.int32)).to(dev)
     dst_t = torch.from_numpy(np.clip(dst, 0, nb).astype(np.int32)).to(dev)
     w_t = torch.from_numpy(w).to(dev)
-    proc_t = torch.from_numpy(proc).to(dev)
+    proc_t = torch.from_numpy(spatial_order(ns, proc)).to(dev)
     dummy_w = torch.zeros(1, dtype=torch.float32, device=dev)
     dummy_e = torch.zeros(1, dtype=torch.uint8, device=dev)
     g = csr.struct(speed)

@@ -40,6 +40,7 @@
 #include "cs_cta.cuh"
 #include "cs_seed.cuh"
 #include "cs_sort.cuh"
+#include "cs_tile.cuh"
 
 namespace cs {
 
@@ -1748,15 +1749,17 @@ Layout layout(int n_bound, int n_slots, int cap, int P, int L, int cta_blocks = 
 // Items that overflowed their slot's capacity run again at 4x the capacity (then 4x again, up to
 // cap = full_n, where nothing can overflow), each level on as many slots as the compact region
 // holds at that capacity; overflows of one level are listed for the next.  `run` launches one
-// level: run(params, slots).  Leaves the last header in h.
+// level: run(params, slots).  first_cap: the first level's capacity where the listed items have not run
+// at the plan's.  Leaves the last header in h.
 template <typename Launch>
 cs_status retry_chain(const cs::PrimalParams &p, const cs_plan *plan, const Layout &lay, char *base, int full_n, int P,
-                      cs::WsHeader &h, cudaStream_t stream, bool poll, Launch run) {
+                      cs::WsHeader &h, cudaStream_t stream, bool poll, Launch run, int first_cap = 0) {
     int32_t *listA = (int32_t *)(base + lay.failed_off);
     int32_t *listB = (int32_t *)(base + lay.failed2_off);
     const int32_t *list = listA;
     unsigned n_in = h.n_failed;
-    int cap_l = (int)std::min<long long>(full_n, 4ll * std::max(plan->cap, 8));
+    int cap_l = first_cap > 0 ? std::min(full_n, first_cap)
+                              : (int)std::min<long long>(full_n, 4ll * std::max(plan->cap, 8));
     while (n_in > 0u) {
         if (n_in > (unsigned)lay.fail_cap) return fail(CS_ERR_CAPACITY, "more overflowed sources than the list holds");
         int32_t *out_l = (list == listA) ? listB : listA;
@@ -1857,6 +1860,27 @@ bool block_schedule(long long n_src) {
     const char *m = getenv("CS_BLOCK_SOURCES_MAX");
     const long long cap = m ? atoll(m) : 4ll * std::max(1, sm_count());
     return n_src <= cap;
+}
+
+// Tile kernel (cs_tile.cu): 32 nearby sources per block, one per lane.  A tile does its sources' common
+// work once, over the union of their reaches, so it pays where the reach is much wider than the tile and
+// there is a tile for every resident block:
+//  - 32 sources for each of the 2 blocks per SM (9,728 on 152 SMs);
+//  - hops to the cutoff (seconds / median edge seconds, half a plan's band width) at least 5 times the
+//    tile's radius sqrt(16 N / sources) in hops.
+// Measured on lattices against one warp per source: 5 km at 80 m (62 hops), every node a source 70 ms
+// against 146 (90,000 nodes), one node in nine 17.5 against 19.6, one in eighteen 16.7 against 12.4;
+// 3.2 km at 100 m (32 hops), every node (19,600) 6.1 against 8.7, every second 4.4 against 5.0, every
+// fourth 4.1 against 3.2; 1.6 km (16 hops) 3.3 against 3.2; 500 m at 80 m 4.8 against 3.5.
+// CS_TILE=0 leaves every source to the other kernels, CS_TILE=1 takes every call the kernel can serve.
+// Returns the sources per tile, 0: not this kernel.
+int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float delta) {
+    const char *e = getenv("CS_TILE");
+    if (e && e[0] == '0') return 0;
+    if (e && e[0] == '1') return (int)std::max(1ll, std::min(32ll, (n_src + blocks - 1) / blocks));
+    if (n_src < 32ll * cs::tile::BPSM * std::max(1, sm_count()) || !(delta > 0.0f)) return 0;
+    const double hops = 2.0 * maxsec / delta, radius = std::sqrt(16.0 * n_bound / (double)n_src);
+    return hops >= 5.0 * radius ? 32 : 0;
 }
 
 // Settle-order sort: distance buckets by default, CS_SORT=radix selects the LSD radix sort.
@@ -1970,6 +1994,72 @@ cs_status reset_dense(char *dense, size_t stride, int n_bound, int n_slots, cuda
     return CS_OK;
 }
 
+// The tile kernel's view of a call.
+cs::tile::Params tile_params(const cs::PrimalParams &p, const Layout &lay, const cs::tile::Geometry &geo, int lanes) {
+    cs::tile::Params c;
+    memset(&c, 0, sizeof(c));
+    const bool od = p.mode == cs::MODE_OD;
+    c.n_bound = p.g.n_bound;
+    c.in_ptr = p.g.in_ptr_dev;
+    c.in_nb = p.g.in_nb_dev;
+    c.in_w = p.g.in_w_dev;
+    c.out_ptr = p.g.out_ptr_dev;
+    c.out_to = p.g.out_to_dev;
+    c.out_w = p.g.out_w_dev;
+    c.out_cnt = p.g.out_cnt_dev;
+    c.node_w = p.g.node_w_dev;
+    c.k = p.k;
+    for (int i = 0; i < p.k; i++) {
+        c.dk[i] = p.dk[i];
+        c.beta[i] = p.beta[i];
+    }
+    c.maxsec = p.maxsec;
+    c.speed = p.speed;
+    c.tol = p.tol;
+    c.delta = p.delta;
+    c.closeness = p.closeness;
+    c.betweenness = p.betweenness;
+    c.track_reach = p.track_reach;
+    c.src_list = p.src_list;
+    c.n_src = p.n_src;
+    c.lanes = lanes;
+    c.src_wt = p.src_wt;
+    c.eligible = od ? nullptr : p.eligible;  // trips carry their own weights
+    c.od_ptr = p.od_ptr;
+    c.od_dst = p.od_dst;
+    c.od_w = p.od_w;
+    c.out = p.out;
+    c.bucket = p.bucket;
+    c.reach = p.reach;
+    c.hdr = p.hdr;
+    c.failed = p.failed;
+    c.fail_cap = p.fail_cap;
+    c.dense = p.dense;
+    c.dense_stride = p.dense_stride;
+    c.aux_off = lay.dense_stride / 2;
+    c.region = p.compact;
+    c.geo = geo;
+    return c;
+}
+
+// Completes a call's rows after its kernels and records its counters (h: the last header read).
+cs_status finish_primal(const cs::PrimalParams &p, const cs::WsHeader &h, bool bucketed, long long n_over,
+                        cudaStream_t stream) {
+    if (bucketed) {
+        const int blocks = std::max(1, std::min((p.g.n_bound + 255) / 256, sm_count() * 8));
+        cs::bucket_prefix_kernel<<<blocks, 256, 0, stream>>>(p.bucket, p.out, p.k, p.g.n_bound);
+        g_counters[3]++;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_fail(e, "bucket_prefix_kernel launch");
+    }
+    g_counters[0] = (long long)h.sources_done;
+    g_counters[1] = (long long)h.edges_relaxed;
+    g_counters[2] = (long long)h.nodes_settled;
+    for (int i = 0; i < 16; i++) cs_host::g_phase[i] = (long long)h.pad[i];
+    cs_set_retries_internal(n_over, 0);
+    return CS_OK;
+}
+
 cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan *plan, void *ws, size_t ws_bytes,
                      cs_outputs out, void *stream_v, int mode, int32_t row_cap, int32_t *t_count, int32_t *t_node,
                      float *t_agg, int32_t *t_pred, const int32_t *tree_src, int32_t n_tree, uint32_t tree_maxsec,
@@ -2066,6 +2156,50 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
         st = launch_seed_table(stream);
         if (st != CS_OK) return st;
     }
+    cs::tile::Geometry geo{};
+    int tile_blocks = 0, lanes = 0;
+    if ((mode == cs::MODE_SHORTEST || mode == cs::MODE_OD) && P <= cs::tile::PMAX) {
+        tile_blocks = std::max(1, std::min(sm_count() * cs::tile::BPSM, plan->n_slots));
+        lanes = tile_lanes(p.n_src, tile_blocks, g->n_bound, p.maxsec, plan->delta_seconds);
+        if (lanes > 0) {
+            tile_blocks = (int)std::min<long long>(tile_blocks, (p.n_src + lanes - 1) / lanes);
+            geo = cs::tile::geometry((lay.compact_total / tile_blocks) & ~size_t(255), K, p.dk, mode == cs::MODE_OD);
+        }
+    }
+    if (geo.mcap >= plan->cap) {
+        // the list of sources left to the per-warp kernel holds fail_cap: more sources run in shares
+        const int64_t n_all = p.n_src;
+        const int32_t *all = p.src_list;
+        long long n_left = 0;
+        cs::WsHeader h;
+        e = cs::tile::launch_seed_table(stream);
+        if (e != cudaSuccess) return cuda_fail(e, "seed table launch");
+        for (int64_t lo = 0; lo < n_all; lo += lay.fail_cap) {
+            p.src_list = all + lo;
+            p.n_src = std::min<int64_t>(n_all - lo, lay.fail_cap);
+            if (lo > 0) {
+                e = cudaMemsetAsync(&p.hdr->work_next, 0, sizeof(unsigned long long), stream);
+                if (e == cudaSuccess) e = cudaMemsetAsync(&p.hdr->n_failed, 0, sizeof(unsigned), stream);
+                if (e != cudaSuccess) return cuda_fail(e, "tile counter reset");
+            }
+            e = cs::tile::launch(tile_params(p, lay, geo, lanes), mode == cs::MODE_OD, tile_blocks, stream);
+            g_counters[3] += 2;
+            if (e != cudaSuccess) return cuda_fail(e, "tile_kernel launch");
+            e = cs::read_header(p.hdr, h, stream, poll);
+            if (e != cudaSuccess) return cuda_fail(e, "tile kernel");
+            if (h.err != 0u)
+                return fail((cs_status)h.err, "device-side check failed (code " + std::to_string(h.err) + " at " +
+                                                  std::to_string(h.err_where) + ")");
+            n_left += h.n_failed;
+            if (h.n_failed > 0u) {
+                st = retry_chain(p, plan, lay, base, g->n_bound, P, h, stream, poll,
+                                 [&](cs::PrimalParams &p2, int slots2) { return launch_primal(p2, plan, slots2, stream); },
+                                 plan->cap);
+                if (st != CS_OK) return st;
+            }
+        }
+        return finish_primal(p, h, bucketed, n_left, stream);
+    }
     if (block) {
         // one block per source with its state on chip; the sources it lists (reach or queues beyond
         // its capacity) run through the per-warp kernel's capacity chain below
@@ -2129,30 +2263,14 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
     if (h.err != 0u)
         return fail((cs_status)h.err, "device-side check failed (code " + std::to_string(h.err) + " at " +
                                           std::to_string(h.err_where) + ")");
-    long long done = (long long)h.sources_done, rel = (long long)h.edges_relaxed, set = (long long)h.nodes_settled;
     const long long n_over = h.n_failed;
     if (h.n_failed > 0u) {
         // Sources whose reach overflowed `cap` (their slots already reset themselves)
         st = retry_chain(p, plan, lay, base, g->n_bound, P, h, stream, poll,
                          [&](cs::PrimalParams &p2, int slots2) { return launch_primal(p2, plan, slots2, stream); });
         if (st != CS_OK) return st;
-        done = (long long)h.sources_done;
-        rel = (long long)h.edges_relaxed;
-        set = (long long)h.nodes_settled;
     }
-    if (bucketed) {
-        int blocks = std::max(1, std::min((g->n_bound + 255) / 256, sm_count() * 8));
-        cs::bucket_prefix_kernel<<<blocks, 256, 0, stream>>>(p.bucket, p.out, K, g->n_bound);
-        g_counters[3]++;
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "bucket_prefix_kernel launch");
-    }
-    g_counters[0] = done;
-    g_counters[1] = rel;
-    g_counters[2] = set;
-    for (int i = 0; i < 16; i++) cs_host::g_phase[i] = (long long)h.pad[i];
-    cs_set_retries_internal(n_over, 0);
-    return CS_OK;
+    return finish_primal(p, h, bucketed, n_over, stream);
 }
 
 cs_status plan_common(int n_bound, int P, int L, int cap, int max_slots, int64_t budget, cs_plan *plan,

@@ -54,14 +54,6 @@ __device__ __forceinline__ dfloat df_two_prod(float a, float b) {
     const float p = __fmul_rn(a, b);
     return {p, __fmaf_rn(a, b, -p)};
 }
-__device__ __forceinline__ dfloat df_add(dfloat a, dfloat b) {
-    dfloat s = df_two_sum(a.h, b.h);
-    const dfloat t = df_two_sum(a.l, b.l);
-    s.l = __fadd_rn(s.l, t.h);
-    s = df_fast_two_sum(s.h, s.l);
-    s.l = __fadd_rn(s.l, t.l);
-    return df_fast_two_sum(s.h, s.l);
-}
 __device__ __forceinline__ dfloat df_mul(dfloat a, dfloat b) {
     dfloat p = df_two_prod(a.h, b.h);
     p.l = __fmaf_rn(a.h, b.l, p.l);
@@ -77,14 +69,15 @@ __device__ __forceinline__ bool seed_exp_df(float beta, float cost, dfloat &r) {
     const int j = min((int)__fmul_rn(y.h, 256.0f), SEED_TAB - 1);
     const dfloat t = df_two_sum(__fsub_rn(y.h, __fmul_rn((float)j, 1.0f / 256.0f)), y.l);
     const float tf = t.h;
-    const float q = __fmul_rn(__fmul_rn(__fmul_rn(tf, tf), tf),
+    const float sq = __fmul_rn(tf, tf), sql = __fmaf_rn(tf, tf, -sq);
+    const float q = __fmul_rn(__fmul_rn(sq, tf),
                               __fmaf_rn(tf, __fmaf_rn(tf, -1.0f / 120.0f, 1.0f / 24.0f), -1.0f / 6.0f));
-    dfloat t2 = df_mul(t, t);
-    t2.h = __fmul_rn(t2.h, 0.5f);
-    t2.l = __fmul_rn(t2.l, 0.5f);
-    dfloat e = df_add({1.0f, 0.0f}, {-t.h, -t.l});
-    e = df_add(e, t2);
-    e = df_add(e, {q, 0.0f});
+    // 1 - t + t^2 / 2 + q: both large steps with their exact errors, the small terms in f32
+    const float s1 = __fsub_rn(1.0f, tf), e1 = __fsub_rn(__fsub_rn(1.0f, s1), tf);
+    const float hh = __fmul_rn(sq, 0.5f);
+    const float s2 = __fadd_rn(s1, hh), e2 = __fsub_rn(hh, __fsub_rn(s2, s1));
+    const float small = __fsub_rn(__fmaf_rn(tf, t.l, __fmaf_rn(0.5f, sql, q)), t.l);
+    const dfloat e = df_fast_two_sum(s2, __fadd_rn(__fadd_rn(e1, e2), small));
     const float2 tj = seed_tab[j];
     r = df_mul({tj.x, tj.y}, e);
     return true;
