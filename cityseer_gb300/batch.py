@@ -201,13 +201,11 @@ class Batch:
                 if jb["betweenness"] and sp.is_source_indexed and sp.n_sources > 0:
                     sc = sp.n_live / sp.n_sources
                     if sc != 1.0:
-                        idx = ns._node_index_array()
-                        data[5][:, idx] *= sc
-                        data[6][:, idx] *= sc
-                res = CentralityShortestResult(jb["d"], ns.node_keys_py(), ns._node_index_array(), data)
+                        data[5:7] *= sc  # removed nodes' entries are zero
+                res = CentralityShortestResult(jb["d"], centrality.node_keys(ns), ns._node_index_array(), data)
                 if sp.is_source_indexed:
                     res.sampled_source_count = sp.sampled_count
             else:
-                res = CentralitySegmentResult(jb["d"], ns.node_keys_py(), ns._node_index_array(), data)
+                res = CentralitySegmentResult(jb["d"], centrality.node_keys(ns), ns._node_index_array(), data)
             out.append(res)
         return out

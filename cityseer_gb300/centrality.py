@@ -63,8 +63,16 @@ class _Result:
             self._idx_list = self._idx.tolist()
         return self._idx_list
 
+    def _load_row(self, m: int, i: int) -> np.ndarray:
+        row = self._data[m, i]
+        return row.copy() if len(self._idx) == len(row) else row[self._idx]  # the indices are unique, ascending
+
     def _load_compact(self, m: int) -> dict[int, np.ndarray]:
-        return {d: self._data[m, i][self._idx].copy() for i, d in enumerate(self.distances)}
+        return {d: self._load_row(m, i) for i, d in enumerate(self.distances)}
+
+    def column(self, name: str, distance: int) -> np.ndarray:
+        """One metric at one distance (what getattr(self, name)[distance] gives, without the others)."""
+        return self._load_row(type(self)._rows.index(name), self.distances.index(distance))
 
     def __getattr__(self, name):
         rows = type(self)._rows
@@ -174,10 +182,12 @@ def prepare_source_sampling(ns, sample_probability, sampling_weights, random_see
         raise ValueError("source_indices and sampling_weights are mutually exclusive")
     exists = a["node_exists"]
     if source_indices is not None:
-        src = np.asarray(list(source_indices), dtype=np.int64)
-        for s in src:
-            if s < 0 or s >= nb or not exists[s]:
-                raise ValueError(f"node index {int(s)} does not exist in the graph")
+        src = np.asarray(source_indices if isinstance(source_indices, np.ndarray) else list(source_indices),
+                         dtype=np.int64).reshape(-1)
+        bad = (src < 0) | (src >= nb)
+        bad[~bad] = ~exists[src[~bad]].astype(bool)
+        if bad.any():
+            raise ValueError(f"node index {int(src[bad][0])} does not exist in the graph")
     n_live = int(live[node_indices].sum())
     is_indexed = source_indices is not None
     sources = src if is_indexed else node_indices
@@ -294,7 +304,7 @@ def spatial_order(ns, process: np.ndarray) -> np.ndarray:
 def drop_device_state(ns, keep_workspace: bool = True) -> None:
     """Forgets the device-resident CSR (and optionally the workspaces) of a graph."""
     for k in list(ns._cache):
-        if k == "primal_csr" or k == "dual_csr" or (not keep_workspace and k in ("ws", "wsd")):
+        if k in ("primal_csr", "dual_csr", "every_source") or (not keep_workspace and k in ("ws", "wsd")):
             del ns._cache[k]
 
 
@@ -409,6 +419,52 @@ def _stream_ptr():
     return torch.cuda.current_stream().cuda_stream
 
 
+def upload(arrays, dev) -> list[torch.Tensor]:
+    """Host arrays as device tensors, through one copy."""
+    at = np.cumsum([0] + [-(-a.nbytes // 16) * 16 for a in arrays])
+    buf = np.empty(int(at[-1]), np.uint8)
+    for a, o in zip(arrays, at):
+        buf[o:o + a.nbytes] = np.ascontiguousarray(a).reshape(-1).view(np.uint8)
+    t = torch.from_numpy(buf).to(dev)
+    return [t[o:o + a.nbytes].view(getattr(torch, a.dtype.name)) for a, o in zip(arrays, at)]
+
+
+def plan_tensors(ns, sp: SourcePlan, process: np.ndarray, dev, order: bool = True) -> list[torch.Tensor]:
+    """The device arrays of a source plan: sources, weights, eligibility.  A call over every live node
+    without sampling depends on the graph alone: its arrays stay with the graph's device state."""
+    every = not sp.is_source_indexed and sp.sample_probability is None and process is sp.process
+    hit = ns._cache.get("every_source") if every else None
+    if hit is not None and hit[0].device == dev:
+        return hit
+    out = upload([spatial_order(ns, process) if order else np.ascontiguousarray(process, np.int32), sp.src_wt,
+                  sp.eligible], dev)
+    if every:
+        ns._cache["every_source"] = out
+    return out
+
+
+def row_buffer(shape, dev) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """(buffer, rows, reach counts): zeroed f64 rows [M][K][N] and u32 counts [K] in one allocation, so
+    that one launch clears them and one copy brings them back."""
+    n = int(np.prod(shape))
+    buf = torch.zeros(n + (shape[1] + 1) // 2, dtype=torch.float64, device=dev)
+    return buf, buf[:n].view(*shape), buf[n:].view(torch.int32)[:shape[1]]
+
+
+def fetch(rows: torch.Tensor, reach: torch.Tensor, buf: torch.Tensor | None) -> tuple[np.ndarray, np.ndarray]:
+    """Host copies of rows and reach counts."""
+    if buf is None:
+        return rows.cpu().numpy(), reach.cpu().numpy()
+    host = buf.cpu().numpy()
+    n = rows.numel()
+    return host[:n].reshape(rows.shape), host[n:].view(np.int32)[:rows.shape[1]]
+
+
+def node_keys(ns) -> list:
+    """The graph's cached key list itself, which nothing changes: results copy it when asked for it."""
+    return ns._cache.get("node_keys") or ns.node_keys_py()
+
+
 # ---------------------------------------------------------------------------------------------
 # centrality_shortest (rust/src/centrality.rs:1624-1874)
 # ---------------------------------------------------------------------------------------------
@@ -426,22 +482,21 @@ def centrality_shortest(ns, distances=None, betas=None, minutes=None, compute_cl
     dists, bets, secs = pair_distances_betas_time(speed, distances, betas, minutes, min_threshold_wt)
     sp = prepare_source_sampling(ns, sample_probability, sampling_weights, random_seed, source_indices)
     track = sp.sample_probability is not None or sp.is_source_indexed
-    rows, reach = shortest_rows(ns, sp, sp.process, dists, bets, secs, speed, tol, closeness, betweenness, track)
-    return finish_shortest(ns, dists, sp, rows.cpu().numpy(), reach.cpu().numpy(), betweenness, track)
+    rows, reach, buf = _shortest_rows(ns, sp, sp.process, dists, bets, secs, speed, tol, closeness, betweenness, track)
+    data, reach_tot = fetch(rows, reach, buf)
+    return finish_shortest(ns, dists, sp, data, reach_tot, betweenness, track)
 
 
 def finish_shortest(ns, dists, sp: SourcePlan, data: np.ndarray, reach_tot: np.ndarray, betweenness: bool,
                     track: bool) -> CentralityShortestResult:
     """Post-scale of betweenness for source subsets (rust/src/centrality.rs:1852-1868) and the
     result object of centrality_shortest."""
-    node_indices = ns._node_index_array()
     if betweenness and sp.is_source_indexed and sp.sample_probability is None and sp.n_sources > 0:
         scale = sp.n_live / sp.n_sources
         if scale != 1.0:
-            data[5][:, node_indices] *= scale
-            data[6][:, node_indices] *= scale
+            data[5:7] *= scale  # removed nodes' entries are zero
     ns._progress = sp.n_sources
-    res = CentralityShortestResult(dists, ns.node_keys_py(), node_indices, data)
+    res = CentralityShortestResult(dists, node_keys(ns), ns._node_index_array(), data)
     if track:
         res.sampled_source_count = sp.sampled_count
         res.reachability_totals = [int(x) for x in reach_tot]
@@ -454,23 +509,27 @@ def shortest_rows(ns, sp: SourcePlan, process: np.ndarray, dists, bets, secs, sp
     eligibility and source weights): ([7][K][N] f64, [K] i64 reach counts) on the graph's device,
     before any post-scale.  The sharded multi-GPU form runs one slice of a plan's sources per rank
     through it."""
+    rows, reach, _ = _shortest_rows(ns, sp, process, dists, bets, secs, speed, tol, closeness, betweenness, track)
+    return rows, reach.to(torch.int64)
+
+
+def _shortest_rows(ns, sp: SourcePlan, process: np.ndarray, dists, bets, secs, speed: float, tol: float,
+                   closeness: bool, betweenness: bool, track: bool):
+    """shortest_rows, and the one buffer that holds rows and counts (None with several launches)."""
     nb = ns.node_bound()
     K = len(dists)
     csr = _primal_csr(ns)
     dev = csr.device
-    proc_t = torch.from_numpy(spatial_order(ns, process)).to(dev)
-    wt_t = torch.from_numpy(sp.src_wt).to(dev)
-    el_t = torch.from_numpy(sp.eligible).to(dev)
+    proc_t, wt_t, el_t = plan_tensors(ns, sp, process, dev)
     g = csr.struct(speed)
     lib = _native.load()
     groups = _groups(K)
     rows = torch.zeros((7, K, nb), dtype=torch.float64, device=dev) if len(groups) > 1 else None
-    reach_all = torch.zeros(K, dtype=torch.int64, device=dev)
+    reach_all = torch.zeros(K, dtype=torch.int64, device=dev) if len(groups) > 1 else None
     for lo, hi in groups:
         k = hi - lo
         ws = _workspace(ns, csr, 0, k, speed, max(secs[lo:hi]))
-        out = torch.zeros((7, k, nb), dtype=torch.float64, device=dev)
-        reach = torch.zeros(k, dtype=torch.int32, device=dev)
+        buf, out, reach = row_buffer((7, k, nb), dev)
         q = _make_query(dists[lo:hi], bets[lo:hi], secs[lo:hi], speed, tol, closeness, betweenness, track,
                         proc_t, wt_t, el_t)
         o = _native.Outputs(out.data_ptr(), reach.data_ptr())
@@ -480,11 +539,10 @@ def shortest_rows(ns, sp: SourcePlan, process: np.ndarray, dists, bets, secs, sp
             ws.init(_stream_ptr())
         _native.check(rc, "cs_centrality_shortest")
         if rows is None:
-            rows = out
-        else:
-            rows[:, lo:hi] = out
+            return out, reach, buf
+        rows[:, lo:hi] = out
         reach_all[lo:hi] = reach.to(torch.int64)
-    return rows, reach_all
+    return rows, reach_all, None
 
 
 # ---------------------------------------------------------------------------------------------
@@ -516,17 +574,14 @@ def betweenness_od_shortest(ns, od_matrix: OdMatrix, distances=None, betas=None,
             raise ValueError(f"OD destination {int(used.max())} is not a node index (node_bound {nb})")
     data = np.zeros((2, K, nb), np.float64)
     ns._progress = len(node_indices)
-    res = BetweennessShortestResult(dists, ns.node_keys_py(), node_indices, data)
+    res = BetweennessShortestResult(dists, node_keys(ns), node_indices, data)
     if not len(proc):
         return res
     csr = _primal_csr(ns)
     dev = csr.device
-    ptr_t = torch.from_numpy(ptr.astype(np.int32)).to(dev)
-    dst_t = torch.from_numpy(np.clip(dst, 0, nb).astype(np.int32)).to(dev)
-    w_t = torch.from_numpy(w).to(dev)
-    proc_t = torch.from_numpy(spatial_order(ns, proc)).to(dev)
-    dummy_w = torch.zeros(1, dtype=torch.float32, device=dev)
-    dummy_e = torch.zeros(1, dtype=torch.uint8, device=dev)
+    ptr_t, dst_t, w_t, proc_t, dummy_w, dummy_e = upload(
+        [ptr.astype(np.int32), np.clip(dst, 0, nb).astype(np.int32), w, spatial_order(ns, proc),
+         np.zeros(1, np.float32), np.zeros(1, np.uint8)], dev)
     g = csr.struct(speed)
     lib = _native.load()
     for lo, hi in _groups(K):
@@ -603,8 +658,8 @@ def segment_rows(ns, process, dists, bets, secs, speed: float, closeness: bool, 
         raise ValueError("Edge not found")
     dev = csr.device
     proc_t = torch.from_numpy(np.ascontiguousarray(process, np.int32)).to(dev)
-    wt_t = torch.zeros(max(nb, 1), dtype=torch.float32, device=dev)
-    el_t = torch.zeros(max(nb, 1), dtype=torch.uint8, device=dev)
+    wt_t = torch.empty(max(nb, 1), dtype=torch.float32, device=dev)  # segments have no source weights
+    el_t = torch.empty(max(nb, 1), dtype=torch.uint8, device=dev)
     g = csr.struct(speed)
     lib = _native.load()
     groups = _cutoff_groups(K)
@@ -631,7 +686,7 @@ def segment_rows(ns, process, dists, bets, secs, speed: float, closeness: bool, 
 def finish_segment(ns, dists, data: np.ndarray) -> CentralitySegmentResult:
     node_indices = ns._node_index_array()
     ns._progress = len(node_indices)
-    return CentralitySegmentResult(dists, ns.node_keys_py(), node_indices, data)
+    return CentralitySegmentResult(dists, node_keys(ns), node_indices, data)
 
 
 # ---------------------------------------------------------------------------------------------

@@ -87,13 +87,18 @@ __device__ __forceinline__ void raise_err(WsHeader *h, unsigned code, unsigned w
 }
 
 // Reads a workspace header after the work queued on `s`.  With poll, waits for the stream by
-// querying it between short sleeps first: a device->host copy into pageable memory issued while
+// querying it first, the first 300 us without sleeping (a sleep overshoots by more than a short call
+// takes: 60-70 us), then between short sleeps: a device->host copy into pageable memory issued while
 // long kernels are still queued holds driver resources until they finish, which stalls other host
 // threads' CUDA calls (allocations, event creation) for that long.
 inline cudaError_t read_header(const WsHeader *dev, WsHeader &h, cudaStream_t s, bool poll) {
     cudaError_t e;
     if (poll) {
-        while ((e = cudaStreamQuery(s)) == cudaErrorNotReady) std::this_thread::sleep_for(std::chrono::microseconds(20));
+        const auto busy_until = std::chrono::steady_clock::now() + std::chrono::microseconds(300);
+        while ((e = cudaStreamQuery(s)) == cudaErrorNotReady) {
+            if (std::chrono::steady_clock::now() < busy_until) std::this_thread::yield();
+            else std::this_thread::sleep_for(std::chrono::microseconds(20));
+        }
         if (e != cudaSuccess) return e;
     }
     e = cudaMemcpyAsync(&h, dev, sizeof(h), cudaMemcpyDeviceToHost, s);

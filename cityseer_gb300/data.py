@@ -77,15 +77,15 @@ class LanduseAccess:
 
     @property
     def weighted(self) -> dict[int, np.ndarray]:
-        return {d: self._w[i][self._idx].copy() for i, d in enumerate(self._d)}
+        return {d: self._w[i][self._idx] for i, d in enumerate(self._d)}
 
     @property
     def unweighted(self) -> dict[int, np.ndarray]:
-        return {d: self._u[i][self._idx].copy() for i, d in enumerate(self._d)}
+        return {d: self._u[i][self._idx] for i, d in enumerate(self._d)}
 
     @property
     def distance(self) -> dict[int, np.ndarray]:
-        return {self._max: self._n[self._idx].copy()}
+        return {self._max: self._n[self._idx]}
 
 
 class AccessibilityResult:
@@ -257,22 +257,17 @@ class DataMap:
         for i, k in enumerate(keys):
             entry_group[i] = groups.setdefault(self.entries[k].dedupe_key, len(groups))
         nb = ns.node_bound()
+        rows = sorted(self.node_data_map.items())
         cnt = np.zeros(nb + 1, np.int64)
-        for node, lst in self.node_data_map.items():
-            cnt[node + 1] = len(lst)
+        nodes = np.array([node for node, _ in rows], np.int64)
+        per = np.array([len(lst) for _, lst in rows], np.int64)
+        cnt[nodes + 1] = per
         ptr = np.cumsum(cnt)
         n_assign = int(ptr[-1])
-        a_entry = np.zeros(n_assign, np.int64)
-        a_dist = np.zeros(n_assign, np.float64)
-        a_node = np.zeros(n_assign, np.int64)
-        a_rank = np.zeros(n_assign, np.int64)
-        for node, lst in self.node_data_map.items():
-            o = int(ptr[node])
-            for r, (k, dd) in enumerate(lst):
-                a_entry[o + r] = pos[k]
-                a_dist[o + r] = dd
-                a_node[o + r] = node
-                a_rank[o + r] = r
+        a_entry = np.array([pos[k] for _, lst in rows for k, _ in lst], np.int64)
+        a_dist = np.array([dd for _, lst in rows for _, dd in lst], np.float64)
+        a_node = np.repeat(nodes, per)
+        a_rank = np.arange(n_assign) - ptr[a_node]
         a_group = entry_group[a_entry] if n_assign else np.zeros(0, np.int64)
         order = np.argsort(a_group, kind="stable")
         gcnt = np.bincount(a_group, minlength=len(groups)) if n_assign else np.zeros(len(groups), np.int64)
@@ -280,8 +275,7 @@ class DataMap:
         gptr[1:] = np.cumsum(gcnt)
         entry_class = np.full(len(keys), -1, np.int64)
         if classes is not None:
-            for i, k in enumerate(keys):
-                entry_class[i] = classes.get(k, -1)
+            entry_class[:] = [classes.get(k, -1) for k in keys]
         return dict(keys=keys, entry_group=entry_group, n_groups=len(groups), ptr=ptr, a_entry=a_entry,
                     a_dist=a_dist, a_node=a_node, a_rank=a_rank, g_ptr=gptr, g_assign=order.astype(np.int64),
                     entry_class=entry_class)
@@ -320,7 +314,8 @@ class DataMap:
             lu[ck] = str(val)
         keys = list(dict.fromkeys(accessibility_keys))
         mcw = np.asarray(common.clip_wts_curve(d, b, int(spatial_tolerance or 0)), np.float32)
-        cls_of = {k: keys.index(v) for k, v in lu.items() if v in keys}
+        place = {v: i for i, v in enumerate(keys)}
+        cls_of = {k: place[v] for k, v in lu.items() if v in place}
         t = self._tables(ns, cls_of)
         nb = ns.node_bound()
         arr = ns.arrays()
@@ -331,10 +326,10 @@ class DataMap:
             from . import access
 
             u, w, n = access.accessibility_rows(ns, t, sources, d, b, s, mcw, speed, len(keys))
-        idx = ns.node_indices()
+        idx = ns._node_index_array()
         res = {key: LanduseAccess(d, idx, w[c], u[c], n[c], max(d)) for c, key in enumerate(keys)}
         self._progress = len(idx)
-        return AccessibilityResult(d, ns.node_keys_py(), idx, res)
+        return AccessibilityResult(d, ns.node_keys_py(), idx.tolist(), res)
 
 
 def _aggregate_host(ns, t, sources, max_seconds: int, speed: float, angular: bool):

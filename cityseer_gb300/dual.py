@@ -212,26 +212,30 @@ def simplest_rows(ns, sp, process, dists, bets, secs, speed, tol, asu, fso, clos
     """The device rows of centrality_simplest for the sources `process` under the plan `sp`:
     ([4][K][N] f64, [K] i64 reach counts) on the graph's device, before any post-scale.  Every
     launch searches to the largest threshold, as the reference's single search does."""
-    from .centrality import _cutoff_groups, _make_query, _stream_ptr
+    rows, reach, _ = _simplest_rows(ns, sp, process, dists, bets, secs, speed, tol, asu, fso, closeness, betweenness,
+                                    track)
+    return rows, reach.to(torch.int64)
+
+
+def _simplest_rows(ns, sp, process, dists, bets, secs, speed, tol, asu, fso, closeness, betweenness, track):
+    """simplest_rows, and the one buffer that holds rows and counts (None with several launches)."""
+    from .centrality import _cutoff_groups, _make_query, _stream_ptr, plan_tensors, row_buffer
 
     nb = ns.node_bound()
     K = len(dists)
     csr = dual_csr(ns)
     dev = csr.device
-    proc_t = torch.from_numpy(np.ascontiguousarray(process, np.int32)).to(dev)
-    wt_t = torch.from_numpy(sp.src_wt).to(dev)
-    el_t = torch.from_numpy(sp.eligible).to(dev)
+    proc_t, wt_t, el_t = plan_tensors(ns, sp, process, dev, order=False)
     g = csr.struct(speed)
     lib = _native.load()
     groups = _cutoff_groups(K)
     rows = torch.zeros((4, K, nb), dtype=torch.float64, device=dev) if len(groups) > 1 else None
-    reach_all = torch.zeros(K, dtype=torch.int64, device=dev)
+    reach_all = torch.zeros(K, dtype=torch.int64, device=dev) if len(groups) > 1 else None
     for lo, hi, sel in groups:
         k = len(sel)
         gd, gb, gs = [dists[i] for i in sel], [bets[i] for i in sel], [secs[i] for i in sel]
         ws = dual_workspace(ns, csr, k, speed, cap=estimate_states(ns, speed, max(gs)))
-        out = torch.zeros((4, k, nb), dtype=torch.float64, device=dev)
-        reach = torch.zeros(k, dtype=torch.int32, device=dev)
+        buf, out, reach = row_buffer((4, k, nb), dev)
         q = _make_query(gd, gb, gs, speed, tol, closeness, betweenness, track, proc_t, wt_t, el_t, asu, fso)
         o = _native.Outputs(out.data_ptr(), reach.data_ptr())
         rc = lib.cs_centrality_simplest(C.byref(g), C.byref(q), C.byref(ws.plan), ws.ptr, ws.nbytes, o, _stream_ptr())
@@ -239,24 +243,22 @@ def simplest_rows(ns, sp, process, dists, bets, secs, speed, tol, asu, fso, clos
             ws.init(_stream_ptr())
         _native.check(rc, "cs_centrality_simplest")
         if rows is None:
-            rows = out
-        else:
-            rows[:, lo:hi] = out[:, : hi - lo]
+            return out, reach, buf
+        rows[:, lo:hi] = out[:, : hi - lo]
         reach_all[lo:hi] = reach[: hi - lo].to(torch.int64)
-    return rows, reach_all
+    return rows, reach_all, None
 
 
 def finish_simplest(ns, dists, sp, data: np.ndarray, reach_tot: np.ndarray, betweenness: bool, track: bool):
     """Post-scale (source subsets) and the result object of centrality_simplest."""
-    from .centrality import CentralitySimplestResult
+    from .centrality import CentralitySimplestResult, node_keys
 
-    node_indices = ns._node_index_array()
     if betweenness and sp.is_source_indexed and sp.sample_probability is None and sp.n_sources > 0:
         scale = sp.n_live / sp.n_sources
         if scale != 1.0:
-            data[3][:, node_indices] *= scale
+            data[3] *= scale  # removed nodes' entries are zero
     ns._progress = sp.n_sources
-    res = CentralitySimplestResult(dists, ns.node_keys_py(), node_indices, data)
+    res = CentralitySimplestResult(dists, node_keys(ns), ns._node_index_array(), data)
     if track:
         res.sampled_source_count = sp.sampled_count
         res.reachability_totals = [int(x) for x in reach_tot]
@@ -265,9 +267,12 @@ def finish_simplest(ns, dists, sp, data: np.ndarray, reach_tot: np.ndarray, betw
 
 def run_simplest(ns, dists, bets, secs, speed, tol, asu, fso, closeness, betweenness, sp):
     track = sp.sample_probability is not None or sp.is_source_indexed
-    rows, reach = simplest_rows(ns, sp, sp.process, dists, bets, secs, speed, tol, asu, fso, closeness, betweenness,
-                                track)
-    return finish_simplest(ns, dists, sp, rows.cpu().numpy(), reach.cpu().numpy(), betweenness, track)
+    from .centrality import fetch
+
+    rows, reach, buf = _simplest_rows(ns, sp, sp.process, dists, bets, secs, speed, tol, asu, fso, closeness,
+                                      betweenness, track)
+    data, reach_tot = fetch(rows, reach, buf)
+    return finish_simplest(ns, dists, sp, data, reach_tot, betweenness, track)
 
 
 class DualTreeWorkspace(device.Workspace):

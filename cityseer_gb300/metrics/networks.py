@@ -85,14 +85,15 @@ def node_centrality_shortest(network_structure, nodes_gdf, distances=None, betas
         for measure, attr in (("beta", "node_beta"), ("cycles", "node_cycles"), ("density", "node_density"),
                               ("farness", "node_farness"), ("harmonic", "node_harmonic")):
             for d, res in results.items():
-                temp[config.prep_gdf_key(measure, d)] = getattr(res, attr)[d]
+                temp[config.prep_gdf_key(measure, d)] = res.column(attr, d)
         for d, res in results.items():
             with np.errstate(divide="ignore", invalid="ignore"):
-                temp[config.prep_gdf_key("hillier", d)] = res.node_density[d] ** 2 / res.node_farness[d]
+                temp[config.prep_gdf_key("hillier", d)] = (temp[config.prep_gdf_key("density", d)] ** 2
+                                                           / temp[config.prep_gdf_key("farness", d)])
     if compute_betweenness:
         for measure, attr in (("betweenness", "node_betweenness"), ("betweenness_beta", "node_betweenness_beta")):
             for d, res in results.items():
-                temp[config.prep_gdf_key(measure, d)] = getattr(res, attr)[d]
+                temp[config.prep_gdf_key(measure, d)] = res.column(attr, d)
     return _write(nodes_gdf, keys, temp)
 
 
@@ -121,14 +122,16 @@ def node_centrality_simplest(network_structure, nodes_gdf, distances=None, betas
     temp = {}
     if compute_closeness:
         for d, res in results.items():
-            temp[config.prep_gdf_key("density", d, angular=True)] = res.node_density[d]
-            temp[config.prep_gdf_key("harmonic", d, angular=True)] = res.node_harmonic[d]
-            temp[config.prep_gdf_key("farness", d, angular=True)] = res.node_farness[d]
+            temp[config.prep_gdf_key("density", d, angular=True)] = res.column("node_density", d)
+            temp[config.prep_gdf_key("harmonic", d, angular=True)] = res.column("node_harmonic", d)
+            temp[config.prep_gdf_key("farness", d, angular=True)] = res.column("node_farness", d)
             with np.errstate(divide="ignore", invalid="ignore"):
-                temp[config.prep_gdf_key("hillier", d, angular=True)] = res.node_density[d] ** 2 / res.node_farness[d]
+                temp[config.prep_gdf_key("hillier", d, angular=True)] = (
+                    temp[config.prep_gdf_key("density", d, angular=True)] ** 2
+                    / temp[config.prep_gdf_key("farness", d, angular=True)])
     if compute_betweenness:
         for d, res in results.items():
-            temp[config.prep_gdf_key("betweenness", d, angular=True)] = res.node_betweenness[d]
+            temp[config.prep_gdf_key("betweenness", d, angular=True)] = res.column("node_betweenness", d)
     return _write(nodes_gdf, keys, temp)
 
 
@@ -145,10 +148,10 @@ def segment_centrality(network_structure, nodes_gdf, distances=None, betas=None,
         for measure, attr in (("seg_density", "segment_density"), ("seg_harmonic", "segment_harmonic"),
                               ("seg_beta", "segment_beta")):
             for d in dists:
-                temp[config.prep_gdf_key(measure, d)] = getattr(res, attr)[d]
+                temp[config.prep_gdf_key(measure, d)] = res.column(attr, d)
     if compute_betweenness is True:
         for d in dists:
-            temp[config.prep_gdf_key("seg_betweenness", d)] = res.segment_betweenness[d]
+            temp[config.prep_gdf_key("seg_betweenness", d)] = res.column("segment_betweenness", d)
     return _write(nodes_gdf, res.node_keys_py, temp)
 
 

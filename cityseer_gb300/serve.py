@@ -109,15 +109,14 @@ class Ticket:
             return self.tree
         data = self.rows.cpu().numpy()
         ns = m["ns"]
-        idx = np.asarray(ns.node_indices(), np.int64)
         if self.query.compute_betweenness and m["n_sources"] > 0:
             sc = m["n_live"] / m["n_sources"]
             if sc != 1.0:
                 for r in m["betw_rows"]:
-                    data[r][:, idx] *= sc
+                    data[r] *= sc  # removed nodes' entries are zero
         cls = {"shortest": CentralityShortestResult, "segment": CentralitySegmentResult,
                "simplest": CentralitySimplestResult}[self.query.mode]
-        res = cls(m["d"], ns.node_keys_py(), ns.node_indices(), data)
+        res = cls(m["d"], centrality.node_keys(ns), ns._node_index_array(), data)
         if self.query.mode != "segment":
             res.sampled_source_count = m["n_sources"]
         return res
