@@ -111,6 +111,7 @@ struct PrimalParams {
     int32_t k;
     float dk[MAXK];
     float beta[MAXK];
+    float inb[MAXK];  // 1 / -beta
     float maxsec;
     float speed;
     float tol;
@@ -835,9 +836,21 @@ __global__ void batch_prefix_kernel(const cs_batch_job *jobs, int n_jobs) {
 // ------------------------------------------------------------------------------------------
 // 4b. Segment centrality for one source.
 // ------------------------------------------------------------------------------------------
+// The shadow term of one half street from a to c: log of c below 1 m, else of the ratio.
+__device__ __forceinline__ float segment_log(float a, float c) {
+    return (a < 1.0f) ? logf(c) : logf(fmaxf(__fdiv_rn(c, a), 1.1920929e-07f));
+}
+
+__device__ __forceinline__ void f64_acc(double &a, float x) { a = __dadd_rn(a, f2d(x)); }
+constexpr int SEG_QUEUE = 160;  // visited streets a warp collects: up to 31 left over and 4 per lane
+constexpr int WORK = BW_COLS * 32 * 12;  // bytes a warp shares: the backward sweep's columns, or the streets
+static_assert(SEG_QUEUE * sizeof(float4) <= WORK, "the streets outgrow the warp's share");
+
 template <int PM>
-CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const SlotPtrs &s, int src, int R) {
+CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const SlotPtrs &s, int src, int R,
+                                                   float4 *queue, long long *ph) {
     const int lane = lane_id();
+    long long tph = clock64();
     const int K = p.k;
     const int N = p.g.n_bound;
     double *const out = (p.mode == MODE_BOTH) ? p.out2 : p.out;  // segment rows
@@ -889,67 +902,118 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
             return;
         }
     }
-    // closeness integrals over visited edges (rust/src/centrality.rs:2201-2317), into the source
-    // thresholds in groups of 4: per lane 12 f64 accumulators in registers and 4 unrolled copies of
-    // the integral code (not 16 of each), one pass over the visited edges per group
+    phase_mark(ph, 2, tph);
+    // closeness integrals over visited edges (rust/src/centrality.rs:2201-2317), into the source's rows;
+    // thresholds in groups of 4, one pass over the visited edges per group.  Bound by the chain of loads
+    // that finds a street's farther end (edge -> neighbour -> its position -> its distance) and by lanes
+    // idle on streets visited from their other end: a lane loads four streets at once, and the visited ones
+    // queue up in shared memory until 32 fill the warp (62,500 sources at 2 km: 19.5 -> 17.9 ms per call,
+    // with one exponential for the middle of both halves and the logs once per street).  Tried and not
+    // faster: sums in pairs of f32 instead of f64 (20.4 ms), the same without the queue (19.5 ms).
     if (p.closeness) for (int kb = 0; kb < K; kb += 4) {
+        const int nk = min(4, K - kb);
+        const float dtop = p.dk[kb + nk - 1];
         double acc[12];
 #pragma unroll
         for (int q = 0; q < 12; q++) acc[q] = 0.0;
-        for (int i = lane; i < R; i += 32) {
-            const int u = s.ord[i];
-            const float au = route_cost(s.sd[i], p.speed);
-            const int beg = __ldg(&p.g.in_ptr_dev[u]);
-            const int end = __ldg(&p.g.in_ptr_dev[u + 1]);
-            for (int e = beg; e < end; e++) {
-                const int nb = __ldg(&p.g.in_nb_dev[e]);
-                float bm;
-                if (nb == u) {
-                    bm = au;
-                } else {
-                    const uint32_t a = s.aux[nb];
-                    if (a > (uint32_t)R) continue;  // cannot happen on clean scratch
-                    if (a != 0u && (int)(a - 1) < i) continue;  // neighbour settled earlier
-                    bm = (a != 0u) ? route_cost(s.sd[a - 1], p.speed) : __int_as_float(INF_BITS);
-                }
-                const bool n_nearer = au <= bm;
-                const float A = n_nearer ? au : bm, Ai = A;
-                const float B = n_nearer ? bm : au, Bi = B;
-                const float elen = __ldg(&p.g.in_seglen_dev[e]);
-                const float imp = __ldg(&p.g.in_segimp_dev[e]);
-                const float C = __fdiv_rn(fadd(fadd(elen, A), B), 2.0f), D = C;
-                const float Ci = fadd(Ai, fmul(__fadd_rn(C, -A), imp)), Di = Ci;
+        int qn = 0;
+        // one visited street per lane: the nearer end at A, the farther at B (inf: not reached)
+        auto integrals = [&](float4 st) {
+            const float A = st.x, B = st.y, elen = st.z, imp = st.w;
+            const float C = fmul(fadd(fadd(elen, A), B), 0.5f);
+            const float Ci = fadd(A, fmul(__fadd_rn(C, -A), imp));
+            const bool two = B != C;
+            float shA = 0.0f, shB = 0.0f;
+            if (C <= dtop) {
+                shA = segment_log(A, Ci);
+                if (two) shB = segment_log(B, Ci);
+            }
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int k = kb + q;
-                    if (k >= K) break;
-                    const float df = p.dk[k];
-                    const float beta = p.beta[k], nbeta = -beta;
-                    const float inb = (beta != 0.0f) ? __fdiv_rn(1.0f, nbeta) : 0.0f;
-                    if (A < df) {
-                        float cc = C, cci = Ci;
-                        if (cc > df) { cc = df; cci = fadd(Ai, fmul(__fadd_rn(df, -A), imp)); }
-                        acc[q] += (double)__fadd_rn(cc, -A);
-                        const float sh = (Ai < 1.0f) ? logf(cci) : logf(fmaxf(__fdiv_rn(cci, Ai), 1.1920929e-07f));
-                        acc[4 + q] += (double)sh;
-                        const float bet = (beta == 0.0f) ? __fadd_rn(cci, -Ai)
-                                                         : fmul(__fadd_rn(expf(fmul(nbeta, cci)), -expf(fmul(nbeta, Ai))), inb);
-                        acc[8 + q] += (double)bet;
+            for (int q = 0; q < 4; q++) {
+                if (q >= nk) break;
+                const int k = kb + q;
+                const float df = p.dk[k];
+                const bool inA = A < df, inB = two && B <= df;
+                if (!inA && !inB) continue;
+                const float beta = p.beta[k], nbeta = -beta, inb = p.inb[k];
+                const bool clip = C > df;
+                const float ec = (clip || beta == 0.0f) ? 0.0f : expf(fmul(nbeta, Ci));  // serves both halves
+                if (inA) {
+                    float cc = C, cci = Ci, sh = shA, e2 = ec;
+                    if (clip) {
+                        cc = df;
+                        cci = fadd(A, fmul(__fadd_rn(df, -A), imp));
+                        sh = segment_log(A, cci);
+                        e2 = expf(fmul(nbeta, cci));
                     }
-                    if (B == D) continue;
-                    if (B <= df) {
-                        float cd = D, cdi = Di;
-                        if (cd > df) { cd = df; cdi = fadd(Bi, fmul(__fadd_rn(df, -B), imp)); }
-                        acc[q] += (double)__fadd_rn(cd, -B);
-                        const float sh = (Bi < 1.0f) ? logf(cdi) : logf(fmaxf(__fdiv_rn(cdi, Bi), 1.1920929e-07f));
-                        acc[4 + q] += (double)sh;
-                        const float bet = (beta == 0.0f) ? __fadd_rn(cdi, -Bi)
-                                                         : fmul(__fadd_rn(expf(fmul(nbeta, cdi)), -expf(fmul(nbeta, Bi))), inb);
-                        acc[8 + q] += (double)bet;
+                    f64_acc(acc[q], __fadd_rn(cc, -A));
+                    f64_acc(acc[4 + q], sh);
+                    f64_acc(acc[8 + q], (beta == 0.0f) ? __fadd_rn(cci, -A)
+                                                       : fmul(__fadd_rn(e2, -expf(fmul(nbeta, A))), inb));
+                }
+                if (inB) {
+                    float cd = C, cdi = Ci, sh = shB, e2 = ec;
+                    if (clip) {
+                        cd = df;
+                        cdi = fadd(B, fmul(__fadd_rn(df, -B), imp));
+                        sh = segment_log(B, cdi);
+                        e2 = expf(fmul(nbeta, cdi));
                     }
+                    f64_acc(acc[q], __fadd_rn(cd, -B));
+                    f64_acc(acc[4 + q], sh);
+                    f64_acc(acc[8 + q], (beta == 0.0f) ? __fadd_rn(cdi, -B)
+                                                       : fmul(__fadd_rn(e2, -expf(fmul(nbeta, B))), inb));
                 }
             }
+        };
+        for (int base = 0; base < R; base += 32) {
+            const int i = base + lane;
+            int u = 0, beg = 0, end = 0;
+            float au = 0.0f;
+            if (i < R) {
+                u = s.ord[i];
+                au = route_cost(s.sd[i], p.speed);
+                if (au <= dtop) {  // no threshold of this group reaches a street from farther on
+                    beg = __ldg(&p.g.in_ptr_dev[u]);
+                    end = __ldg(&p.g.in_ptr_dev[u + 1]);
+                }
+            }
+            const int most = warp_max_i(end - beg);
+            for (int j0 = 0; j0 < most; j0 += 4) {
+                // four streets' loads at once: neighbour, its position, its distance
+                int nb[4];
+                uint32_t at[4];
+                float B[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) nb[j] = (beg + j0 + j < end) ? __ldg(&p.g.in_nb_dev[beg + j0 + j]) : -1;
+#pragma unroll
+                for (int j = 0; j < 4; j++) at[j] = (nb[j] >= 0 && nb[j] != u) ? s.aux[nb[j]] : 0u;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    B[j] = (at[j] != 0u && at[j] <= (uint32_t)R) ? route_cost(s.sd[at[j] - 1], p.speed)
+                                                                 : __int_as_float(INF_BITS);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    // visited from here: a self loop, or a neighbour not settled earlier
+                    const bool take = nb[j] >= 0 && (nb[j] == u || at[j] == 0u || ((int)(at[j] - 1) >= i && at[j] <= (uint32_t)R));
+                    const unsigned m = __ballot_sync(FULL, take);
+                    if (take) {
+                        const int e = beg + j0 + j;
+                        queue[qn + __popc(m & lanemask_lt())] =
+                            make_float4(au, nb[j] == u ? au : B[j], __ldg(&p.g.in_seglen_dev[e]), __ldg(&p.g.in_segimp_dev[e]));
+                    }
+                    qn += __popc(m);
+                }
+                __syncwarp();
+                while (qn >= 32) {
+                    qn -= 32;
+                    integrals(queue[qn + lane]);
+                }
+                __syncwarp();
+            }
         }
+        if (lane < qn) integrals(queue[lane]);
+        __syncwarp();
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const int k = kb + q;
@@ -964,6 +1028,7 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
             }
         }
     }
+    phase_mark(ph, 3, tph);
     if (!p.betweenness) return;
     // betweenness: subtree sums of per-target auc (rust/src/centrality.rs:2319-2401)
     double *acc = s.dl;  // [R][K]
@@ -988,8 +1053,7 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
                 const float sdist = route_cost(s.sd[i], p.speed);
                 const float o_len = s.fb[i], l_len = s.fa[i];
                 const float min_span = __fadd_rn(__fadd_rn(sdist, -o_len), -l_len);
-                const float o_1 = min_span, o_2 = fadd(min_span, o_len);
-                const float l_1 = min_span, l_2 = fadd(min_span, l_len);
+                const float o_2 = fadd(min_span, o_len), l_2 = fadd(min_span, l_len);
                 const bool own = (i > 0) && (v > src);
                 for (int k = 0; k < K; k++) {
                     const double below = __ldcg(&acc[(size_t)i * K + k]);
@@ -1000,17 +1064,20 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
                         if (min_span <= df) {
                             const float o2s = fminf(o_2, df), l2s = fminf(l_2, df);
                             float auc;
-                            if (beta == 0.0f) auc = fadd(__fadd_rn(o2s, -o_1), __fadd_rn(l2s, -l_1));
+                            if (beta == 0.0f) auc = fadd(__fadd_rn(o2s, -min_span), __fadd_rn(l2s, -min_span));
                             else {
-                                const float nb = -beta, inb = __fdiv_rn(1.0f, nb);
-                                auc = fadd(fmul(__fadd_rn(expf(fmul(nb, o2s)), -expf(fmul(nb, o_1))), inb),
-                                           fmul(__fadd_rn(expf(fmul(nb, l2s)), -expf(fmul(nb, l_1))), inb));
+                                const float nb = -beta, inb = p.inb[k];
+                                const float e1 = expf(fmul(nb, min_span));  // both segments start at the span
+                                auc = fadd(fmul(__fadd_rn(expf(fmul(nb, o2s)), -e1), inb),
+                                           fmul(__fadd_rn(expf(fmul(nb, l2s)), -e1), inb));
                             }
-                            if (isfinite(auc) && auc >= 0.0f) total += (double)auc;
+                            if (isfinite(auc) && auc > 0.0f) total = __dadd_rn(total, f2d(auc));
                         }
                     }
-                    if (i > 0 && v != src && below > 0.0) atomicAdd(out + ((size_t)3 * K + k) * N + v, below);
-                    if (pp >= 0 && total != 0.0) atomicAdd(&acc[(size_t)pp * K + k], total);
+                    // sums of terms >= 0: their bits tell zero from more without the f64 pipe
+                    if (i > 0 && v != src && __double_as_longlong(below) > 0ll)
+                        atomicAdd(out + ((size_t)3 * K + k) * N + v, below);
+                    if (pp >= 0 && __double_as_longlong(total) != 0ll) atomicAdd(&acc[(size_t)pp * K + k], total);
                 }
                 mine = true;
             }
@@ -1023,6 +1090,7 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
             return;
         }
     }
+    phase_mark(ph, 5, tph);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1166,20 +1234,20 @@ __device__ __forceinline__ bool run_source(const PrimalParams &p, const SlotPtrs
     if constexpr (MODE == MODE_SHORTEST) {
         shortest_accumulate<PM, 0>(p, s, src, R, ph, cnt, bw_pl, bw_fr);
     } else if constexpr (MODE == MODE_SEGMENT) {
-        segment_accumulate<PM>(p, s, src, R);
+        segment_accumulate<PM>(p, s, src, R, (float4 *)bw_fr, ph);
     } else if constexpr (MODE == MODE_TREE) {
         tree_rows<PM>(p, s, li, R);
     } else if constexpr (MODE == MODE_OD) {
         shortest_accumulate<PM, 0, true>(p, s, src, R, ph, cnt, bw_pl, bw_fr);
     } else {
         if (p.mode == MODE_SHORTEST) shortest_accumulate<PM, 0>(p, s, src, R, ph, cnt, bw_pl, bw_fr);
-        else if (p.mode == MODE_SEGMENT) segment_accumulate<PM>(p, s, src, R);
+        else if (p.mode == MODE_SEGMENT) segment_accumulate<PM>(p, s, src, R, (float4 *)bw_fr, ph);
         else if (p.mode == MODE_BOTH) {
             // one search and settle order serve both: shortest rows, then segment rows (its own
             // single-predecessor replay over the same positions)
             shortest_accumulate<PM, 0>(p, s, src, R, ph, cnt, bw_pl, bw_fr);
             __syncwarp();
-            segment_accumulate<PM>(p, s, src, R);
+            segment_accumulate<PM>(p, s, src, R, (float4 *)bw_fr, ph);
         } else tree_rows<PM>(p, s, li, R);
     }
     __syncwarp();
@@ -1215,7 +1283,7 @@ __device__ __forceinline__ void flush_counters(const PrimalParams &p, long long 
 // meets (a warp without a source, or whose source overflowed, runs the phases empty).
 template <int PM>
 __device__ __forceinline__ bool run_segment_sync(const PrimalParams &p, const SlotPtrs &s, bool mine, int li, int src,
-                                                 uint32_t *hist, long long *ph, long long &relaxed,
+                                                 uint32_t *hist, float4 *queue, long long *ph, long long &relaxed,
                                                  long long &settled) {
     const int lane = lane_id();
     long long t0 = clock64();
@@ -1246,7 +1314,7 @@ __device__ __forceinline__ bool run_segment_sync(const PrimalParams &p, const Sl
     phase_mark(ph, 1, t0);
     __syncthreads();
     if (live) {
-        segment_accumulate<PM>(p, s, src, R);
+        segment_accumulate<PM>(p, s, src, R, queue, ph);
         __syncwarp();
         t0 = clock64();
         for (int i = lane; i < R; i += 32) {
@@ -1265,6 +1333,7 @@ __device__ __forceinline__ bool run_segment_sync(const PrimalParams &p, const Sl
 template <int PM, int MINB>
 __global__ void __launch_bounds__(256, MINB) segment_sync_kernel(const PrimalParams p) {
     __shared__ uint32_t hist_all[8][256];
+    __shared__ float4 queue_all[8][SEG_QUEUE];
     __shared__ long long ph_all[8][8];
     __shared__ unsigned long long blk_base;
     __shared__ unsigned blk_err;
@@ -1293,7 +1362,7 @@ __global__ void __launch_bounds__(256, MINB) segment_sync_kernel(const PrimalPar
         const bool mine = has_slot && idx < (unsigned long long)p.n_src;
         const int li = mine ? (p.remap ? p.remap[idx] : (int)idx) : 0;
         const int src = mine ? p.src_list[li] : 0;
-        if (run_segment_sync<PM>(p, s, mine, li, src, hist_all[wib], ph, relaxed, settled)) {
+        if (run_segment_sync<PM>(p, s, mine, li, src, hist_all[wib], queue_all[wib], ph, relaxed, settled)) {
             done_src++;
             if (lane == 0) count_progress(p.hdr);
         }
@@ -1306,9 +1375,9 @@ __global__ void __launch_bounds__(256, MINB) primal_kernel(const PrimalParams p)
     __shared__ uint32_t hist_all[8][256];
     __shared__ int cnt_all[8][4 * MAXK + 2];
     __shared__ long long ph_all[8][8];
-    // backward sweep: each lane's predecessor rows and sigma fractions (column-major per warp)
-    __shared__ int bw_pl_all[8][bw_cols(PM) * 32];
-    __shared__ double bw_fr_all[8][bw_cols(PM) * 32];
+    // per warp: the backward sweep's columns (each lane's sigma fractions and predecessor rows), or the
+    // visited streets of the segment integrals
+    __shared__ __align__(16) double work_all[8][WORK / 8];
     const int lane = lane_id();
     const int wib = threadIdx.x >> 5;
     const int slot = (int)((blockIdx.x * (blockDim.x >> 5)) + wib);
@@ -1325,8 +1394,8 @@ __global__ void __launch_bounds__(256, MINB) primal_kernel(const PrimalParams p)
         if (idx >= (unsigned long long)p.n_src) break;
         if (__ldcg(&p.hdr->err) != 0u) break;
         const int li = p.remap ? p.remap[idx] : (int)idx;
-        if (run_source<PM, MODE>(p, s, li, p.src_list[li], hist_all[wib], cnt_all[wib], bw_pl_all[wib], bw_fr_all[wib],
-                                 ph, relaxed, settled)) {
+        if (run_source<PM, MODE>(p, s, li, p.src_list[li], hist_all[wib], cnt_all[wib],
+                                 (int *)(work_all[wib] + bw_cols(PM) * 32), work_all[wib], ph, relaxed, settled)) {
             done_src++;
             if (lane == 0) count_progress(p.hdr);
         }
@@ -1447,6 +1516,7 @@ __device__ __forceinline__ void job_params(const PrimalParams &base, const cs_ba
     for (int i = 0; i < MAXK; i++) {
         p.dk[i] = i < j.k ? (float)j.distances[i] : 0.0f;
         p.beta[i] = i < j.k ? j.betas[i] : 0.0f;
+        p.inb[i] = __fdiv_rn(1.0f, -p.beta[i]);
         if (i < j.k) maxs = max(maxs, j.seconds[i]);
     }
     p.maxsec = (float)maxs;
@@ -1474,9 +1544,9 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const PrimalParams bas
     __shared__ uint32_t hist_all[8][256];
     __shared__ int cnt_all[8][4 * MAXK + 2];
     __shared__ long long ph_all[8][8];
-    // backward sweep: each lane's predecessor rows and sigma fractions (column-major per warp)
-    __shared__ int bw_pl_all[8][bw_cols(PM) * 32];
-    __shared__ double bw_fr_all[8][bw_cols(PM) * 32];
+    // per warp: the backward sweep's columns (each lane's sigma fractions and predecessor rows), or the
+    // visited streets of the segment integrals
+    __shared__ __align__(16) double work_all[8][WORK / 8];
     const int lane = lane_id();
     const int wib = threadIdx.x >> 5;
     const int slot = (int)((blockIdx.x * (blockDim.x >> 5)) + wib);
@@ -1509,8 +1579,8 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const PrimalParams bas
         }
         const int li = (int)(item - jobs[jb].item_begin);
         // failures record the global item index
-        if (run_source<PM, MODE>(p, s, (int)item, p.src_list[li], hist_all[wib], cnt_all[wib], bw_pl_all[wib],
-                                 bw_fr_all[wib], ph, relaxed, settled)) {
+        if (run_source<PM, MODE>(p, s, (int)item, p.src_list[li], hist_all[wib], cnt_all[wib],
+                                 (int *)(work_all[wib] + bw_cols(PM) * 32), work_all[wib], ph, relaxed, settled)) {
             done_src++;
             if (lane == 0) count_progress(base.hdr);
         }
@@ -1518,16 +1588,16 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const PrimalParams bas
     flush_counters(base, ph, relaxed, settled, done_src);
 }
 
-// Batched shortest-path items with block-synchronous phases (as primal_sync_kernel): a block
-// claims one item per warp; each warp looks its item's job up.  Every warp reaches every barrier.
-template <int PM, int MINB>
+// Batched shortest-path or segment items with block-synchronous phases (as primal_sync_kernel and
+// segment_sync_kernel): a block claims one item per warp; each warp looks its item's job up.  Every warp
+// reaches every barrier.
+template <int PM, int MINB, int MODE>
 __global__ void __launch_bounds__(256, MINB) batch_sync_kernel(const PrimalParams base, const cs_batch_job *jobs,
                                                                int n_jobs, long long item_lo, long long item_hi) {
     __shared__ uint32_t hist_all[8][256];
     __shared__ int cnt_all[8][4 * MAXK + 2];
     __shared__ long long ph_all[8][8];
-    __shared__ int bw_pl_all[8][bw_cols(PM) * 32];
-    __shared__ double bw_fr_all[8][bw_cols(PM) * 32];
+    __shared__ __align__(16) double work_all[8][WORK / 8];
     __shared__ long long blk_base;
     __shared__ unsigned blk_err;
     const int lane = lane_id();
@@ -1601,8 +1671,12 @@ __global__ void __launch_bounds__(256, MINB) batch_sync_kernel(const PrimalParam
         __syncthreads();
         // every warp of the block runs the phases with the same closeness / betweenness flags
         // only when its jobs agree on them; the barrier count must not depend on the job
-        shortest_accumulate<PM, 8>(p, s, ok ? src : 0, ok ? R : 0, ph, cnt_all[wib], bw_pl_all[wib],
-                                   bw_fr_all[wib]);
+        if constexpr (MODE == MODE_SEGMENT) {
+            if (ok) segment_accumulate<PM>(p, s, src, R, (float4 *)work_all[wib], ph);
+        } else {
+            shortest_accumulate<PM, 8>(p, s, ok ? src : 0, ok ? R : 0, ph, cnt_all[wib],
+                                       (int *)(work_all[wib] + bw_cols(PM) * 32), work_all[wib]);
+        }
         __syncwarp();
         t0 = clock64();
         if (ok) {
@@ -1948,6 +2022,14 @@ void launch_batch_mode(const cs::PrimalParams &p, int minb, int blocks, const cs
     }
 }
 
+template <int MODE>
+void launch_batch_sync(const cs::PrimalParams &p, int minb, int blocks, const cs_batch_job *jobs_dev, int n_jobs,
+                       long long lo, long long hi, cudaStream_t stream) {
+    if (minb == 4) cs::batch_sync_kernel<8, 4, MODE><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, lo, hi);
+    else if (minb == 3) cs::batch_sync_kernel<8, 3, MODE><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, lo, hi);
+    else cs::batch_sync_kernel<8, 2, MODE><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, lo, hi);
+}
+
 // mode: the jobs' common mode (0 or 1) for a mode-specialised kernel, else -1
 cs_status launch_batch(cs::PrimalParams &p, const cs_plan *plan, const cs_batch_job *jobs_dev, int n_jobs,
                        long long item_lo, long long item_hi, int n_slots, int mode, cudaStream_t stream) {
@@ -1960,9 +2042,9 @@ cs_status launch_batch(cs::PrimalParams &p, const cs_plan *plan, const cs_batch_
     }
     p.n_slots = n_slots;
     if (mode == cs::MODE_SHORTEST && p.P <= 8 && !p.rerun && phase_sync()) {
-        if (minb == 4) cs::batch_sync_kernel<8, 4><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, item_lo, item_hi);
-        else if (minb == 3) cs::batch_sync_kernel<8, 3><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, item_lo, item_hi);
-        else cs::batch_sync_kernel<8, 2><<<blocks, 256, 0, stream>>>(p, jobs_dev, n_jobs, item_lo, item_hi);
+        launch_batch_sync<cs::MODE_SHORTEST>(p, minb, blocks, jobs_dev, n_jobs, item_lo, item_hi, stream);
+    } else if (mode == cs::MODE_SEGMENT && p.P <= 8 && !p.rerun && phase_sync()) {
+        launch_batch_sync<cs::MODE_SEGMENT>(p, minb, blocks, jobs_dev, n_jobs, item_lo, item_hi, stream);
     } else if (mode == cs::MODE_SHORTEST)
         launch_batch_mode<cs::MODE_SHORTEST>(p, minb, blocks, jobs_dev, n_jobs, item_lo, item_hi, stream);
     else if (mode == cs::MODE_SEGMENT)
@@ -2098,6 +2180,7 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
         for (int i = 0; i < K; i++) {
             p.dk[i] = (float)q->distances[i];
             p.beta[i] = q->betas[i];
+            p.inb[i] = 1.0f / -p.beta[i];
             maxs = std::max(maxs, q->seconds[i]);
         }
         p.speed = q->speed_m_s;
