@@ -19,9 +19,10 @@ BUILD_DIR = PKG_DIR / "_build"
 LIB_PATH = BUILD_DIR / "libcsgpu.so"
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
-CUDA_SOURCES = ["cs_primal.cu", "cs_dual.cu", "cs_cta.cu", "cs_tile.cu"]
+CUDA_SOURCES = ["cs_primal_batch.cu", "cs_dual.cu", "cs_cta.cu", "cs_tile.cu", "cs_primal_shortest.cu",
+                "cs_primal_segment.cu", "cs_primal_tree.cu", "cs_primal.cu"]
 CXX_SOURCES = ["cs_host.cpp"]
-HEADERS = ["cs_common.cuh", "cs_sort.cuh", "cs_seed.cuh", "cs_cta.cuh", "cs_tile.cuh"]
+HEADERS = ["cs_common.cuh", "cs_primal.cuh", "cs_sort.cuh", "cs_seed.cuh", "cs_cta.cuh", "cs_tile.cuh"]
 
 
 def _nvcc() -> str:
