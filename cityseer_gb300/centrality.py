@@ -309,7 +309,7 @@ def drop_device_state(ns, keep_workspace: bool = True) -> None:
 
 
 def estimate_reach(ns, csr, speed: float, max_seconds: int, n_samples: int = 48) -> int:
-    """Largest reach (nodes settled) over an even sample of sources, from the tree kernel run with
+    """Largest reach (nodes settled) over a spread sample of sources, from the tree kernel run with
     one-wide rows (it then reports only the count)."""
     key = ("reach", float(np.float32(speed)), int(max_seconds))
     hit = ns._cache.get(key)
@@ -318,7 +318,10 @@ def estimate_reach(ns, csr, speed: float, max_seconds: int, n_samples: int = 48)
     idx = ns._node_index_array()
     if len(idx) == 0:
         return 1
-    pick = idx[np.linspace(0, len(idx) - 1, min(n_samples, len(idx))).astype(np.int64)]
+    # golden-ratio steps: even ones can fall on one column of a lattice (its edge, of half the reach)
+    n = min(n_samples, len(idx))
+    at = np.arange(n) if n == len(idx) else (np.arange(n) * 0.6180339887498949 % 1.0 * len(idx)).astype(np.int64)
+    pick = idx[at]
     lib = _native.load()
     plan = device.plan_primal(csr, 2, 1, speed, cap=csr.n_bound, max_slots=len(pick))
     ws = device.Workspace(plan, csr.n_bound, csr.device)
