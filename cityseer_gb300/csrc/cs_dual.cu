@@ -13,7 +13,8 @@
 // each state's chosen route.  Per source, one warp:
 //  A. Label-correcting search over states: atomicMin on a packed (route, seconds) 64-bit key gives
 //     the lexicographic least fixpoint, route first.
-//  B. Warp radix sort of the reached states by route: the reference's settle order.
+//  B. Warp sort of the reached states by route (route buckets, re-sorts by radix): the reference's
+//     settle order.
 //  C. Replay, in route order, of every state's candidate offers through the reference's tie rules:
 //     final route, seconds, predecessors and sigma, each checked bit for bit against A.  The tie
 //     window can make the reference keep seconds that differ from the lexicographic minimum; a
@@ -43,7 +44,22 @@ constexpr unsigned long long KEY_INF = 0xffffffffffffffffull;
 // The key of a reached state whose every offer was withdrawn (a NaN route, above every real key and
 // below KEY_INF): it offers nothing, a new offer replaces it, and it is not reached a second time.
 constexpr unsigned long long KEY_WITHDRAWN = KEY_INF - 2ull;
-constexpr int DPM = 8;  // max incoming / outgoing dual edges per state handled in registers
+constexpr int DPM = 8;  // max incoming / outgoing dual edges per dual node
+// Each state has the edges of one end of its street, half of its dual node's: the packed records list a
+// node's edges of slot 0 first (cs_dual_pack), so a state's lie in the first or the last W of them.  W = 4
+// serves graphs whose states have at most 4 (intersections of degree 5), W = 8 every other (42,465 sources
+// at 2 km: 105.8 ms against 139.4 with 8 records per state); cs_dual_pack
+// marks the latter in the sign of the first forward record's seconds, and both kernels are launched, the
+// one that the mark does not name ending at once (2-3 us, without a host read of the mark).
+__device__ __forceinline__ float rec_secs(const uint4 &ed) { return fabsf(__uint_as_float(ed.y)); }
+__device__ __forceinline__ bool wide_states(const cs_dual_graph &g) {
+    return g.n_edges > 0 && (((const uint4 *)g.fwd_pack_dev)->y >> 31) != 0u;
+}
+// The window of W records that holds the edges of slot `side` among [beg, end).
+template <int W>
+__device__ __forceinline__ int side_window(int beg, int end, int side) {
+    return side ? max(beg, end - W) : beg;
+}
 
 __host__ __device__ inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -220,7 +236,8 @@ __device__ __noinline__ unsigned long long dual_rekey(const DualParams &p, const
     return best;
 }
 
-__device__ int dual_search(const DualParams &p, const DSlot &s, int src, long long &relaxed) {
+template <int W>
+__device__ int dual_search(const DualParams &p, const DSlot &s, int src, long long &relaxed, float &rmax) {
     const float maxsec_ = p.maxsec, delta_ = p.delta;  // in registers (p may live in shared memory)
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
@@ -266,11 +283,12 @@ __device__ int dual_search(const DualParams &p, const DSlot &s, int src, long lo
                 // a first touch's entry knows the state's discovery index; later entries look it up
                 const uint32_t aS = (live && qi == 0u) ? __ldcg(&s.aux[S]) : qi;
                 const int u = S >> 1, e = S & 1;
-                const int beg = live ? __ldg(&p.g.ptr_dev[u]) : 0;
-                const int deg = live ? __ldg(&p.g.ptr_dev[u + 1]) - beg : 0;
+                const int e0 = live ? __ldg(&p.g.ptr_dev[u]) : 0, e1 = live ? __ldg(&p.g.ptr_dev[u + 1]) : 0;
+                const int beg = side_window<W>(e0, e1, 1 - e);
+                const int deg = min(e1 - e0, W);
                 const bool track = live && aS != 0u && aS <= (uint32_t)cap;
                 const unsigned long long lk = track ? __ldcg(&lastk[aS - 1]) : KEY_INF;
-                relaxed += deg;
+                relaxed += e1 - e0;
                 const float rU = hi_f(kS), sU = lo_f(kS);
                 const float rL = hi_f(lk), sL = lo_f(lk);
                 // withdrawals only from a state relaxing again (it has a last key), within the budget
@@ -286,7 +304,7 @@ __device__ int dual_search(const DualParams &p, const DSlot &s, int src, long lo
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         const uint4 ed = (j0 + q < deg) ? __ldg(&fe[beg + j0 + q]) : make_uint4(0u, 0u, 0u, 0u);
-                        const float cs_ = __fadd_rn(sU, __uint_as_float(ed.y));
+                        const float cs_ = __fadd_rn(sU, rec_secs(ed));
                         const bool ok = j0 + q < deg && (int)(ed.x >> 31) == 1 - e && cs_ <= maxsec_;
                         Vq[q] = (int)(ed.x & 0x7fffffffu);
                         crq[q] = cand_route(rU, __uint_as_float(ed.z), __uint_as_float(ed.w));
@@ -303,7 +321,7 @@ __device__ int dual_search(const DualParams &p, const DSlot &s, int src, long lo
                         if (again && !imp && j0 + q < deg) {
                             // the offer this edge carried at the state's last relaxation (record re-read)
                             const uint4 ed = __ldg(&fe[beg + j0 + q]);
-                            const float ocs = __fadd_rn(sL, __uint_as_float(ed.y));
+                            const float ocs = __fadd_rn(sL, rec_secs(ed));
                             if ((int)(ed.x >> 31) == 1 - e && ocs <= maxsec_) {
                                 const unsigned long long ok =
                                     pack(cand_route(rL, __uint_as_float(ed.z), __uint_as_float(ed.w)), ocs);
@@ -361,6 +379,7 @@ __device__ int dual_search(const DualParams &p, const DSlot &s, int src, long lo
         nfar = nf2;
     }
     __syncwarp();
+    rmax = T;  // the last band's end
     if (overflow) return -1;
     return R;
 }
@@ -380,7 +399,7 @@ __device__ int dual_search(const DualParams &p, const DSlot &s, int src, long lo
 constexpr uint32_t NO_LSEC = 0xffffffffu;
 constexpr unsigned long long NO_KEY = KEY_INF - 1ull;  // a NaN route: never a key
 
-__device__ int dual_search_wide(const DualParams &p, const DSlot &s, int src, long long &relaxed) {
+__device__ int dual_search_wide(const DualParams &p, const DSlot &s, int src, long long &relaxed, float &rmax) {
     const float maxsec_ = p.maxsec, delta_ = p.delta;  // in registers (p may live in shared memory)
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
@@ -429,7 +448,7 @@ __device__ int dual_search_wide(const DualParams &p, const DSlot &s, int src, lo
                     if (j < deg) {
                         const uint4 ed = __ldg((const uint4 *)p.g.fwd_pack_dev + beg + j);
                         if ((int)(ed.x >> 31) == 1 - e) {
-                            const float w = __uint_as_float(ed.y);
+                            const float w = rec_secs(ed);
                             const float cs_ = has_key ? __fadd_rn(sU, w) : __int_as_float(INF_BITS);
                             // a key's path is a path too: lsec stays <= the key's seconds
                             const float ls_ = fminf(__fadd_rn(lU, w), cs_);
@@ -506,6 +525,7 @@ __device__ int dual_search_wide(const DualParams &p, const DSlot &s, int src, lo
         nfar = nf2;
     }
     __syncwarp();
+    rmax = T;  // the last band's end
     if (overflow) return -1;
     return R;
 }
@@ -623,31 +643,35 @@ __device__ int dual_exact_search(const DualParams &p, const DSlot &s, int src) {
 // ------------------------------------------------------------------------------------------
 // C. Replay in route order.
 // ------------------------------------------------------------------------------------------
+template <int W>
 struct DOff {
-    int pos[DPM];
-    float cr[DPM];
-    float cs[DPM];
+    int pos[W];
+    float cr[W];
+    float cs[W];
     unsigned valid;  // offers settled before the target
 };
 
-__device__ __forceinline__ int dnext(const DOff &o, unsigned todo) {
+template <int W>
+__device__ __forceinline__ int dnext(const DOff<W> &o, unsigned todo) {
     int best = -1, bp = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < DPM; j++)
+    for (int j = 0; j < W; j++)
         if (((todo >> j) & 1u) && o.pos[j] < bp) { bp = o.pos[j]; best = j; }
     return best;
 }
 
-__device__ __forceinline__ bool dpos_in(const DOff &o, unsigned mask, int pos) {
+template <int W>
+__device__ __forceinline__ bool dpos_in(const DOff<W> &o, unsigned mask, int pos) {
     bool has = false;
 #pragma unroll
-    for (int j = 0; j < DPM; j++) has |= ((mask >> j) & 1u) && o.pos[j] == pos;
+    for (int j = 0; j < W; j++) has |= ((mask >> j) & 1u) && o.pos[j] == pos;
     return has;
 }
 
 // Reference state machine (rust/src/centrality.rs:658-693) over offers in settle order; returns the
 // predecessor mask and writes the replayed route and seconds.
-__device__ __forceinline__ unsigned dreplay(const DualParams &p, const DOff &o, float &route, float &secs) {
+template <int W>
+__device__ __forceinline__ unsigned dreplay(const DualParams &p, const DOff<W> &o, float &route, float &secs) {
     const float one_plus = 1.0f + TIE_EPSILON, one_minus = 1.0f - TIE_EPSILON;
     float cur = __int_as_float(INF_BITS), sc = __int_as_float(INF_BITS);
     unsigned pm = 0u, t = o.valid;
@@ -657,7 +681,7 @@ __device__ __forceinline__ unsigned dreplay(const DualParams &p, const DOff &o, 
         float crj = 0.0f, csj = 0.0f;
         int pj = 0;
 #pragma unroll
-        for (int q = 0; q < DPM; q++)
+        for (int q = 0; q < W; q++)
             if (q == j) { crj = o.cr[q]; csj = o.cs[q]; pj = o.pos[q]; }
         if (csj > p.maxsec) continue;
         const bool improved = crj < cur;
@@ -684,7 +708,7 @@ __device__ __forceinline__ unsigned dreplay(const DualParams &p, const DOff &o, 
             float crj = 0.0f;
             int pj = 0;
 #pragma unroll
-            for (int q = 0; q < DPM; q++)
+            for (int q = 0; q < W; q++)
                 if (q == j) { crj = o.cr[q]; pj = o.pos[q]; }
             if (crj <= lim && !dpos_in(o, pm, pj)) pm |= 1u << j;
         }
@@ -693,48 +717,49 @@ __device__ __forceinline__ unsigned dreplay(const DualParams &p, const DOff &o, 
 }
 
 // The replay keeps each state's offers (position, or -1; route; seconds) for the node-level best,
-// in the search queues' space (free once the search is done): 8 positions in qa, 8 routes in qb,
-// 8 seconds in qf per settle position.
-__device__ __forceinline__ void store_doffers(const DSlot &s, int i, const DOff &o) {
-    int4 *op = (int4 *)s.qa + 2 * (size_t)i;
-    float4 *cp = (float4 *)s.qb + 2 * (size_t)i;
-    float4 *sp = (float4 *)s.qf + 2 * (size_t)i;
-    int q[DPM];
+// in the search queues' space (free once the search is done): W positions in qa, W routes in qb,
+// W seconds in qf per settle position.
+template <int W>
+__device__ __forceinline__ void store_doffers(const DSlot &s, int i, const DOff<W> &o) {
 #pragma unroll
-    for (int j = 0; j < DPM; j++) q[j] = ((o.valid >> j) & 1u) ? o.pos[j] : -1;
-    op[0] = make_int4(q[0], q[1], q[2], q[3]);
-    op[1] = make_int4(q[4], q[5], q[6], q[7]);
-    cp[0] = make_float4(o.cr[0], o.cr[1], o.cr[2], o.cr[3]);
-    cp[1] = make_float4(o.cr[4], o.cr[5], o.cr[6], o.cr[7]);
-    sp[0] = make_float4(o.cs[0], o.cs[1], o.cs[2], o.cs[3]);
-    sp[1] = make_float4(o.cs[4], o.cs[5], o.cs[6], o.cs[7]);
+    for (int h = 0; h < W / 4; h++) {
+        const size_t at = (size_t)(W / 4) * i + h;
+        int q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) q[j] = ((o.valid >> (4 * h + j)) & 1u) ? o.pos[4 * h + j] : -1;
+        ((int4 *)s.qa)[at] = make_int4(q[0], q[1], q[2], q[3]);
+        ((float4 *)s.qb)[at] = make_float4(o.cr[4 * h], o.cr[4 * h + 1], o.cr[4 * h + 2], o.cr[4 * h + 3]);
+        ((float4 *)s.qf)[at] = make_float4(o.cs[4 * h], o.cs[4 * h + 1], o.cs[4 * h + 2], o.cs[4 * h + 3]);
+    }
 }
 
-__device__ __forceinline__ void load_doffers(const DSlot &s, int i, DOff &o) {
-    const int4 *op = (const int4 *)s.qa + 2 * (size_t)i;
-    const float4 *cp = (const float4 *)s.qb + 2 * (size_t)i;
-    const float4 *sp = (const float4 *)s.qf + 2 * (size_t)i;
-    const int4 a = __ldcg(op), b = __ldcg(op + 1);
-    const float4 c = __ldcg(cp), d = __ldcg(cp + 1), e = __ldcg(sp), f = __ldcg(sp + 1);
-    const int q[DPM] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    const float cr[DPM] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
-    const float cs[DPM] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
+template <int W>
+__device__ __forceinline__ void load_doffers(const DSlot &s, int i, DOff<W> &o) {
     o.valid = 0u;
 #pragma unroll
-    for (int j = 0; j < DPM; j++) {
-        o.pos[j] = q[j];
-        o.cr[j] = cr[j];
-        o.cs[j] = cs[j];
-        if (q[j] >= 0) o.valid |= 1u << j;
+    for (int h = 0; h < W / 4; h++) {
+        const size_t at = (size_t)(W / 4) * i + h;
+        const int4 a = __ldcg((const int4 *)s.qa + at);
+        const float4 c = __ldcg((const float4 *)s.qb + at), e = __ldcg((const float4 *)s.qf + at);
+        const int q[4] = {a.x, a.y, a.z, a.w};
+        const float cr[4] = {c.x, c.y, c.z, c.w}, cs[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            o.pos[4 * h + j] = q[j];
+            o.cr[4 * h + j] = cr[j];
+            o.cs[4 * h + j] = cs[j];
+            if (q[j] >= 0) o.valid |= 1u << (4 * h + j);
+        }
     }
 }
 
 // Node-level best route / seconds (rust/src/centrality.rs:695-703) over offers to both states of
 // the node, in the global settle order of the offering states.  Positions of the states: i0/i1
 // (-1 when unreached).
+template <int W>
 __device__ __forceinline__ void node_best(const DualParams &p, const DSlot &s, int v, int src, int i0, int i1, int R,
                                           float &best, float &bsecs, bool &bad) {
-    DOff o0, o1;
+    DOff<W> o0, o1;
     o0.valid = 0u;
     o1.valid = 0u;
     if (i0 >= 0) load_doffers(s, i0, o0);
@@ -749,7 +774,7 @@ __device__ __forceinline__ void node_best(const DualParams &p, const DSlot &s, i
         int p0 = 0x7fffffff, p1 = 0x7fffffff;
         float c0 = 0.0f, s0 = 0.0f, c1 = 0.0f, s1 = 0.0f;
 #pragma unroll
-        for (int q = 0; q < DPM; q++) {
+        for (int q = 0; q < W; q++) {
             if (q == j0) { p0 = o0.pos[q]; c0 = o0.cr[q]; s0 = o0.cs[q]; }
             if (q == j1) { p1 = o1.pos[q]; c1 = o1.cr[q]; s1 = o1.cs[q]; }
         }
@@ -783,6 +808,7 @@ __device__ __forceinline__ int first_ks(const DualParams &p, float secs) {
 // reach a state the search did not.
 // check_reach: run the reach check even when every replayed value equals its key (the keys were
 // rewritten by an earlier round, and the search never relaxed from the rewritten seconds).
+template <int W>
 __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, bool &bad, bool rewrite,
                            bool check_reach, int start, int &first_change) {
     const int lane = lane_id();
@@ -802,24 +828,25 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
         // The state's offers from reached states settled before it: positions and dual edges, found
         // once; the offer values need the offerers' replayed route and seconds, final once the
         // in-chunk offerers (pm) are done.
-        DOff o;
+        DOff<W> o;
         o.valid = 0u;
         unsigned pm = 0u;
         const uint4 *re = (const uint4 *)p.g.rev_pack_dev;
         int rbeg = 0;  // the state's incoming records: re[rbeg + j]
         if (act && !is_src) {
             const int v = V >> 1, sv = V & 1;
-            rbeg = __ldg(&p.g.rptr_dev[v]);
-            const int deg = min(__ldg(&p.g.rptr_dev[v + 1]) - rbeg, DPM);
-            uint32_t aa[DPM];
+            const int r0 = __ldg(&p.g.rptr_dev[v]), r1 = __ldg(&p.g.rptr_dev[v + 1]);
+            rbeg = side_window<W>(r0, r1, sv);
+            const int deg = min(r1 - r0, W);
+            uint32_t aa[W];
 #pragma unroll
-            for (int j = 0; j < DPM; j++) {
+            for (int j = 0; j < W; j++) {
                 aa[j] = 0u;
                 const unsigned x = (j < deg) ? __ldg(&re[rbeg + j]).x : 0u;
                 if (j < deg && (int)(x >> 31) == sv) aa[j] = s.aux[x & 0x7fffffffu];
             }
 #pragma unroll
-            for (int j = 0; j < DPM; j++) {
+            for (int j = 0; j < W; j++) {
                 o.pos[j] = -1;
                 if (aa[j] > (uint32_t)R) bad = true;
                 if (aa[j] != 0u && aa[j] <= (uint32_t)R && (int)aa[j] - 1 < i) {
@@ -831,7 +858,7 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < DPM; j++) {
+            for (int j = 0; j < W; j++) {
                 o.pos[j] = -1;
                 o.cr[j] = 0.0f;
                 o.cs[j] = 0.0f;
@@ -852,7 +879,7 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
                     sg = 1.0;
                 } else {
 #pragma unroll
-                    for (int j = 0; j < DPM; j++) {
+                    for (int j = 0; j < W; j++) {
                         o.cr[j] = 0.0f;
                         o.cs[j] = 0.0f;
                         if ((o.valid >> j) & 1u) {
@@ -862,10 +889,10 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
                             o.cs[j] = __fadd_rn(__ldcg(&s.sB[pu]), __uint_as_float(ed.y));
                         }
                     }
-                const unsigned pmask = dreplay(p, o, route, secs);
+                    const unsigned pmask = dreplay<W>(p, o, route, secs);
                     sg = 0.0;
 #pragma unroll
-                    for (int j = 0; j < DPM; j++) {
+                    for (int j = 0; j < W; j++) {
                         if ((pmask >> j) & 1u) {
                             s.pr[(size_t)i * DPM + np] = o.pos[j];
                             sg = __dadd_rn(sg, s.sig[o.pos[j]]);
@@ -877,7 +904,7 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
                 s.sB[i] = secs;
                 s.sig[i] = sg;
                 s.np[i] = (uint8_t)np;
-                store_doffers(s, i, o);
+                store_doffers<W>(s, i, o);
                 const unsigned long long k = __ldcg(&s.key[V]);
                 // a widened-pass state without a key that the replay leaves unreached agrees
                 const bool both_unreached = (k == KEY_INF || k == KEY_WITHDRAWN) && route == __int_as_float(INF_BITS);
@@ -956,10 +983,11 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
         const int u = U >> 1, e = U & 1;
         const float sU = s.sB[i];
         const int beg = __ldg(&p.g.ptr_dev[u]), end = __ldg(&p.g.ptr_dev[u + 1]);
-        for (int ej = beg; ej < end; ej++) {
+        const int w0 = side_window<W>(beg, end, 1 - e);
+        for (int ej = w0; ej < min(end, w0 + W); ej++) {
             const uint4 ed = __ldg((const uint4 *)p.g.fwd_pack_dev + ej);
             if ((int)(ed.x >> 31) != 1 - e) continue;
-            if (__fadd_rn(sU, __uint_as_float(ed.y)) > p.maxsec) continue;
+            if (__fadd_rn(sU, rec_secs(ed)) > p.maxsec) continue;
             const int V = (int)(ed.x & 0x7fffffffu);
             const uint32_t a = s.aux[V];
             if (a == 0u) escape = true;
@@ -980,6 +1008,12 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
 // ------------------------------------------------------------------------------------------
 // D + E. Node best, closeness, backward sweep.
 // ------------------------------------------------------------------------------------------
+// Comparisons of the f64 values here (>= 0, finite) by their bits: no use of the f64 pipe, which GB300
+// runs at 1/64 of the f32 rate.
+__device__ __forceinline__ bool is_zero(double x) { return __double_as_longlong(x) == 0ll; }
+__device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
+
+template <int W>
 __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, int R, int *cnt, bool &bad, long long *ph) {
     long long tph = clock64();
     const int lane = lane_id();
@@ -1004,7 +1038,7 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
         const int i0 = (V & 1) ? isib : i;
         const int i1 = (V & 1) ? i : isib;
         float best, bsecs;
-        node_best(p, s, v, src, i0, i1, R, best, bsecs, bad);
+        node_best<W>(p, s, v, src, i0, i1, R, best, bsecs, bad);
         s.nbR[i] = best;
         s.nbS[i] = bsecs;
         if (isib >= 0) {
@@ -1048,10 +1082,10 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
         const int i = base + lane;
         const bool act = i < R;
         const int np = act ? s.np[i] : 0;
-        int pl[DPM];
+        int pl[W];
         unsigned pm = 0u;
 #pragma unroll
-        for (int r = 0; r < DPM; r++) {
+        for (int r = 0; r < W; r++) {
             pl[r] = (r < np) ? s.pr[(size_t)i * DPM + r] : 0;
             if (r < np && pl[r] >= base) pm |= 1u << (pl[r] - base);
         }
@@ -1076,42 +1110,42 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
                 const float route_sib = isib >= 0 ? s.rB[isib] : 0.0f;
                 const double pair = (inf >> 31) ? 0.5 : 1.0;
                 // predecessor factors sigma_v / sigma_w in f64 (1 exactly when the counts agree)
-                double fr[DPM];
+                double fr[W];
 #pragma unroll
-                for (int r = 0; r < DPM; r++) {
+                for (int r = 0; r < W; r++) {
                     fr[r] = 0.0;
                     if (r < np) {
                         const double sv = s.sig[pl[r]];
-                        fr[r] = (sv == sw) ? 1.0 : __ddiv_rn(sv, sw);
+                        fr[r] = same_bits(sv, sw) ? 1.0 : __ddiv_rn(sv, sw);
                     }
                 }
                 double *dli = dl + (size_t)i * K;
                 for (int k = 0; k < K; k++) {
                     const float thr = p.sk[k];
                     if (!(secs <= thr)) continue;  // include_state: agg_seconds <= threshold
-                    if (sw == 0.0) continue;
+                    if (is_zero(sw)) continue;
                     double seed = 0.0;
                     if (v != src && isfinite(best) && isfinite(bsecs) && bsecs <= thr) {
-                        const bool me = sw != 0.0 && secs <= thr && route <= __fmul_rn(best, one_tol);
-                        const bool sib = isib >= 0 && sig_sib != 0.0 && secs_sib <= thr &&
+                        const bool me = !is_zero(sw) && secs <= thr && route <= __fmul_rn(best, one_tol);
+                        const bool sib = isib >= 0 && !is_zero(sig_sib) && secs_sib <= thr &&
                                          route_sib <= __fmul_rn(best, one_tol);
                         if (me) {
                             // the seed splits the pair count over the best states by sigma
                             // (rust/src/centrality.rs:2066-2077), in f64
                             const double tot = sib ? __dadd_rn(sw, sig_sib) : sw;
-                            seed = (tot == sw) ? pair : __dmul_rn(pair, __ddiv_rn(sw, tot));
+                            seed = same_bits(tot, sw) ? pair : __dmul_rn(pair, __ddiv_rn(sw, tot));
                         }
                     }
                     const double dep = __dadd_rn(seed, __ldcg(&dli[k]));
-                    if (dep == 0.0) continue;
+                    if (is_zero(dep)) continue;
 #pragma unroll
-                    for (int r = 0; r < DPM; r++) {
-                        if (r >= np || fr[r] == 0.0) continue;
-                        atomicAdd(&dl[(size_t)pl[r] * K + k], fr[r] == 1.0 ? dep : __dmul_rn(fr[r], dep));
+                    for (int r = 0; r < W; r++) {
+                        if (r >= np || is_zero(fr[r])) continue;
+                        atomicAdd(&dl[(size_t)pl[r] * K + k], same_bits(fr[r], 1.0) ? dep : __dmul_rn(fr[r], dep));
                     }
                     if (v == src) continue;
                     const double credit = __dadd_rn(dep, -seed);
-                    if (credit > 0.0)
+                    if (__double_as_longlong(credit) > 0ll)
                         atomicAdd(p.out + ((size_t)3 * K + k) * N + v, unit_wt ? credit : __dmul_rn(credit, wtd));
                 }
                 mine = true;
@@ -1134,6 +1168,7 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
 // One source on this warp's slot: search, settle order, replay, accumulation, scratch reset.
 // Returns true when the source was accumulated; false when it was listed (overflow or a replay
 // that disagreed) for a later pass.  li is what the lists record.
+template <int W>
 __device__ __forceinline__ bool run_dual_source(const DualParams &p, const DSlot &s, int li, int src, uint32_t *hist,
                                                 int *cnt, long long *ph, long long &relaxed, long long &settled) {
     const int lane = lane_id();
@@ -1142,12 +1177,13 @@ __device__ __forceinline__ bool run_dual_source(const DualParams &p, const DSlot
     const bool exact = (p.pass == 2) || p.force_exact;
     const bool wide = s.lsec != nullptr;
     int R;
+    float rmax = 0.0f;  // above every reached route
     if (exact) {
         R = dual_exact_search(p, s, src);
     } else if (wide) {
-        R = dual_search_wide(p, s, src, relaxed);
+        R = dual_search_wide(p, s, src, relaxed, rmax);
     } else {
-        R = dual_search(p, s, src, relaxed);
+        R = dual_search<W>(p, s, src, relaxed, rmax);
     }
     dphase(ph, exact ? 6 : 0, tph);
     if (R < 0) {
@@ -1185,7 +1221,7 @@ __device__ __forceinline__ bool run_dual_source(const DualParams &p, const DSlot
         int start = 0;
         if (!exact) {
             if (it == 0) {
-                warp_radix_sort(R, s.rl, key_of, s.kb, s.vb, s.rk, s.ord, hist);
+                warp_bucket_sort(R, rmax, s.rl, key_of, s.kb, s.vb, s.rk, s.ord, hist);
             } else {
                 // Only the keys the last round rewrote changed, and no state ahead of first_change
                 // moves: the suffix from there is sorted again (from its current order, which holds
@@ -1217,14 +1253,14 @@ __device__ __forceinline__ bool run_dual_source(const DualParams &p, const DSlot
         __syncwarp();
         dphase(ph, 1, tph);
         // after a round that rewrote keys, lower rewritten seconds may reach states the search cut
-        rr = dual_replay(p, s, src, R, bad, !exact, it > 0, start, first_change);
+        rr = dual_replay<W>(p, s, src, R, bad, !exact, it > 0, start, first_change);
         __syncwarp();
         dphase(ph, 2, tph);
     }
     if (lane == 0) ph[7] += rounds_run;
     const bool ok = rr == 0;
     if (ok) {
-        dual_accumulate(p, s, src, R, cnt, bad, ph);
+        dual_accumulate<W>(p, s, src, R, cnt, bad, ph);
         tph = clock64();
     } else if (lane == 0) {
         if (exact) raise_err(p.hdr, CS_ERR_INTERNAL, 24);  // the exact pass must replay cleanly
@@ -1252,6 +1288,7 @@ __device__ __forceinline__ bool run_dual_source(const DualParams &p, const DSlot
 // then accumulation + scratch reset, each phase closed by a block barrier that every warp meets
 // (a warp without a source, or whose source overflowed, runs the phases empty), so that the SM
 // fetches one phase's code at a time.  Returns true when the source was accumulated.
+template <int W>
 __device__ __forceinline__ bool run_dual_source_sync(const DualParams &p, const DSlot &s, bool mine, int li,
                                                      int src, uint32_t *hist, int *cnt, long long *ph,
                                                      long long &relaxed, long long &settled) {
@@ -1261,10 +1298,11 @@ __device__ __forceinline__ bool run_dual_source_sync(const DualParams &p, const 
     const bool exact = (p.pass == 2) || p.force_exact;
     const bool wide = s.lsec != nullptr;
     int R = 0;
+    float rmax = 0.0f;  // above every reached route
     if (mine) {
         if (exact) R = dual_exact_search(p, s, src);
-        else if (wide) R = dual_search_wide(p, s, src, relaxed);
-        else R = dual_search(p, s, src, relaxed);
+        else if (wide) R = dual_search_wide(p, s, src, relaxed, rmax);
+        else R = dual_search<W>(p, s, src, relaxed, rmax);
     }
     dphase(ph, exact ? 6 : 0, tph);
     __syncthreads();
@@ -1299,7 +1337,7 @@ __device__ __forceinline__ bool run_dual_source_sync(const DualParams &p, const 
             int start = 0;
             if (!exact) {
                 if (it == 0) {
-                    warp_radix_sort(R, s.rl, key_of, s.kb, s.vb, s.rk, s.ord, hist);
+                    warp_bucket_sort(R, rmax, s.rl, key_of, s.kb, s.vb, s.rk, s.ord, hist);
                 } else {
                     const int p0 = max(0, min(first_change, R));
                     for (int i = p0 + lane; i < R; i += 32) prev[i] = s.ord[i];
@@ -1325,7 +1363,7 @@ __device__ __forceinline__ bool run_dual_source_sync(const DualParams &p, const 
             for (int i = start + lane; i < R; i += 32) s.aux[s.ord[i]] = (uint32_t)(i + 1);
             __syncwarp();
             dphase(ph, 1, tph);
-            rr = dual_replay(p, s, src, R, bad, !exact, it > 0, start, first_change);
+            rr = dual_replay<W>(p, s, src, R, bad, !exact, it > 0, start, first_change);
             __syncwarp();
             dphase(ph, 2, tph);
         }
@@ -1336,7 +1374,7 @@ __device__ __forceinline__ bool run_dual_source_sync(const DualParams &p, const 
     const bool ok = live && rr == 0;
     if (live) {
         if (ok) {
-            dual_accumulate(p, s, src, R, cnt, bad, ph);
+            dual_accumulate<W>(p, s, src, R, cnt, bad, ph);
             tph = clock64();
         } else if (lane == 0) {
             if (exact) raise_err(p.hdr, CS_ERR_INTERNAL, 24);
@@ -1377,8 +1415,9 @@ __device__ __forceinline__ void flush_dual_counters(const DualParams &p, const l
 
 // dual_kernel with the block's warps in lockstep (run_dual_source_sync): a block claims one source per
 // warp at a time; every warp of the block stays in the loop until the block's sources run out.
-template <int MINB>
+template <int MINB, int W>
 __global__ void __launch_bounds__(256, MINB) dual_sync_kernel(const DualParams p) {
+    if (wide_states(p.g) != (W == DPM)) return;
     __shared__ uint32_t hist_all[8][256];
     __shared__ int cnt_all[8][MAXK];
     __shared__ long long ph_all[8][16];
@@ -1410,7 +1449,7 @@ __global__ void __launch_bounds__(256, MINB) dual_sync_kernel(const DualParams p
         const bool mine = has_slot && idx < (unsigned long long)p.n_src;
         const int li = mine ? (p.remap ? p.remap[idx] : (int)idx) : 0;
         const int src = mine ? p.src_list[li] : 0;
-        if (run_dual_source_sync(p, s, mine, li, src, hist_all[wib], cnt_all[wib], ph, relaxed, settled)) {
+        if (run_dual_source_sync<W>(p, s, mine, li, src, hist_all[wib], cnt_all[wib], ph, relaxed, settled)) {
             done_src++;
             if (lane == 0) count_progress(p.hdr);
         }
@@ -1418,8 +1457,9 @@ __global__ void __launch_bounds__(256, MINB) dual_sync_kernel(const DualParams p
     if (has_slot) flush_dual_counters(p, ph, relaxed, settled, done_src);
 }
 
-template <int MINB>
+template <int MINB, int W>
 __global__ void __launch_bounds__(256, MINB) dual_kernel(const DualParams p) {
+    if (wide_states(p.g) != (W == DPM)) return;
     __shared__ uint32_t hist_all[8][256];
     __shared__ int cnt_all[8][MAXK];
     __shared__ long long ph_all[8][16];
@@ -1440,7 +1480,7 @@ __global__ void __launch_bounds__(256, MINB) dual_kernel(const DualParams p) {
         if (idx >= (unsigned long long)p.n_src) break;
         if (__ldcg(&p.hdr->err) != 0u) break;
         const int li = p.remap ? p.remap[idx] : (int)idx;
-        if (run_dual_source(p, s, li, p.src_list[li], hist_all[wib], cnt_all[wib], ph, relaxed, settled)) {
+        if (run_dual_source<W>(p, s, li, p.src_list[li], hist_all[wib], cnt_all[wib], ph, relaxed, settled)) {
             done_src++;
             if (lane_id() == 0) count_progress(p.hdr);
         }
@@ -1523,7 +1563,7 @@ __global__ void __launch_bounds__(256, MINB) dual_batch_kernel(const DualParams 
             cur_job = jb;
         }
         const int li = (int)(item - jobs[jb].item_begin);
-        if (run_dual_source(p, s, (int)item, p.src_list[li], hist_all[wib], cnt_all[wib], ph, relaxed, settled))
+        if (run_dual_source<DPM>(p, s, (int)item, p.src_list[li], hist_all[wib], cnt_all[wib], ph, relaxed, settled))
             done_src++;
     }
     flush_dual_counters(base, ph, relaxed, settled, done_src);
@@ -1735,16 +1775,38 @@ __global__ void __launch_bounds__(256) dual_tree_kernel(const DTreeParams p) {
     }
 }
 
-// Packed edge records (one 128-bit load per edge in the searches and the replay).
+// Packed edge records (one 128-bit load per edge in the searches and the replay), one thread per dual
+// node: within each node's range the edges of slot 0 first, each slot's in list order.
 __global__ void dual_pack_kernel(const cs_dual_graph g, uint4 *fwd, uint4 *rev) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < g.n_edges; e += gridDim.x * blockDim.x) {
-        const unsigned ex = g.exit_slot_dev[e], en = g.entry_slot_dev[e];
-        fwd[e] = make_uint4((unsigned)(2 * g.to_dev[e]) + en | (ex << 31), __float_as_uint(g.w_dev[e]),
-                            __float_as_uint(g.ang_dev[e]), __float_as_uint(g.len_dev[e]));
-        const int id = g.rid_dev[e];
-        const unsigned rex = g.exit_slot_dev[id], ren = g.entry_slot_dev[id];
-        rev[e] = make_uint4((unsigned)(2 * g.rfrom_dev[e]) + (1u - rex) | (ren << 31), __float_as_uint(g.w_dev[id]),
-                            __float_as_uint(g.ang_dev[id]), __float_as_uint(g.len_dev[id]));
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n_bound; v += gridDim.x * blockDim.x) {
+        for (int side = 0, o = g.ptr_dev[v]; side < 2; side++) {
+            for (int e = g.ptr_dev[v]; e < g.ptr_dev[v + 1]; e++) {
+                const unsigned ex = g.exit_slot_dev[e], en = g.entry_slot_dev[e];
+                if ((int)ex != side) continue;
+                fwd[o++] = make_uint4((unsigned)(2 * g.to_dev[e]) + en | (ex << 31), __float_as_uint(g.w_dev[e]),
+                                      __float_as_uint(g.ang_dev[e]), __float_as_uint(g.len_dev[e]));
+            }
+        }
+        for (int side = 0, o = g.rptr_dev[v]; side < 2; side++) {
+            for (int e = g.rptr_dev[v]; e < g.rptr_dev[v + 1]; e++) {
+                const int id = g.rid_dev[e];
+                const unsigned rex = g.exit_slot_dev[id], ren = g.entry_slot_dev[id];
+                if ((int)ren != side) continue;
+                rev[o++] = make_uint4((unsigned)(2 * g.rfrom_dev[e]) + (1u - rex) | (ren << 31),
+                                      __float_as_uint(g.w_dev[id]), __float_as_uint(g.ang_dev[id]),
+                                      __float_as_uint(g.len_dev[id]));
+            }
+        }
+    }
+}
+
+// Marks the records of a graph with more than 4 edges at one end of a street (after dual_pack_kernel).
+__global__ void dual_mark_kernel(const cs_dual_graph g, uint4 *fwd, const uint4 *rev) {
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n_bound; v += gridDim.x * blockDim.x) {
+        int out[2] = {0, 0}, in[2] = {0, 0};
+        for (int e = g.ptr_dev[v]; e < g.ptr_dev[v + 1]; e++) out[fwd[e].x >> 31]++;
+        for (int e = g.rptr_dev[v]; e < g.rptr_dev[v + 1]; e++) in[rev[e].x >> 31]++;
+        if (max(max(out[0], out[1]), max(in[0], in[1])) > 4) atomicOr(&fwd[0].y, 0x80000000u);
     }
 }
 
@@ -1885,13 +1947,18 @@ int dual_wide_mode() {
     return 1;
 }
 
-// Resident 256-thread blocks per SM the dual kernels are compiled for: 4 (32 warps per SM, 64
-// registers).  On the 124,500-node curved dual the memory latency the extra warps hide outweighs their
-// register spills: 224k sources/s at 2 km against 211k with 3 blocks (30.9k and 30.4k at 5 km); 3
-// blocks had beaten 2 by 5% and 8%.  CS_DUAL_MINB=2 or 3 selects the other builds.
-int dual_minb() {
+// Resident 256-thread blocks per SM that plans are sized for and the wide kernels (W = 8) run with: 4 (32
+// warps per SM, 64 registers).  On the 124,500-node curved dual the memory latency the extra warps hide
+// outweighs their register spills: 224k sources/s at 2 km against 211k with 3 blocks (30.9k and 30.4k
+// at 5 km); 3 blocks had beaten 2 by 5% and 8%.  The narrow kernels (W = 4) run with 3: 42,465 sources
+// at 2 km took 95.3 ms against 99.2 with 4.  CS_DUAL_MINB=2, 3 or 4 selects one build for both.
+int requested_dual_minb() {
     const char *e = getenv("CS_DUAL_MINB");
-    return (e && e[0] == '2') ? 2 : ((e && e[0] == '3') ? 3 : 4);
+    return (e && e[0] >= '2' && e[0] <= '4') ? e[0] - '0' : 0;
+}
+int dual_minb() {
+    const int v = requested_dual_minb();
+    return v ? v : 4;
 }
 
 // Lockstep phases for the simplest-path kernel (default; CS_DUAL_SYNC=0 leaves each warp on its own
@@ -1902,15 +1969,25 @@ bool dual_sync() {
     return !(e && e[0] == '0');
 }
 
+template <int MINB, int W>
+void dlaunch_width(csd::DualParams p, cudaStream_t s) {
+    // a tighter build than the plan's slots were sized for: the blocks that are resident at once
+    const int blocks = std::max(1, std::min((p.n_slots + 7) / 8, std::max(1, dsm_count()) * MINB));
+    p.n_slots = std::min(p.n_slots, blocks * 8);
+    if (dual_sync()) csd::dual_sync_kernel<MINB, W><<<blocks, 256, 0, s>>>(p);
+    else csd::dual_kernel<MINB, W><<<blocks, 256, 0, s>>>(p);
+}
+
 cs_status dlaunch(csd::DualParams &p, int n_slots, cudaStream_t s) {
     p.n_slots = n_slots;
-    if (dual_sync()) {
-        if (dual_minb() == 4) csd::dual_sync_kernel<4><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
-        else if (dual_minb() == 3) csd::dual_sync_kernel<3><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
-        else csd::dual_sync_kernel<2><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
-    } else if (dual_minb() == 4) csd::dual_kernel<4><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
-    else if (dual_minb() == 3) csd::dual_kernel<3><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
-    else csd::dual_kernel<2><<<(n_slots + 7) / 8, 256, 0, s>>>(p);
+    // both widths: the graph's mark names the one that runs
+    const int v = requested_dual_minb();
+    if (v == 4) dlaunch_width<4, 4>(p, s);
+    else if (v == 2) dlaunch_width<2, 4>(p, s);
+    else dlaunch_width<3, 4>(p, s);
+    if (v == 3) dlaunch_width<3, csd::DPM>(p, s);
+    else if (v == 2) dlaunch_width<2, csd::DPM>(p, s);
+    else dlaunch_width<4, csd::DPM>(p, s);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CS_OK : dcuda(e, "dual_kernel launch");
 }
@@ -2023,8 +2100,9 @@ cs_status cs_dual_pack(const cs_dual_graph *g, void *fwd_pack_dev, void *rev_pac
     if (!fwd_pack_dev || !rev_pack_dev) return dfail(CS_ERR_ARG, "packed record arrays are NULL");
     if (((uintptr_t)fwd_pack_dev | (uintptr_t)rev_pack_dev) & 15u)
         return dfail(CS_ERR_ARG, "packed edge records must be 16-byte aligned");
-    const int blocks = std::max(1, std::min((g->n_edges + 255) / 256, std::max(1, dsm_count()) * 8));
+    const int blocks = std::max(1, std::min((g->n_bound + 255) / 256, std::max(1, dsm_count()) * 8));
     csd::dual_pack_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(*g, (uint4 *)fwd_pack_dev, (uint4 *)rev_pack_dev);
+    csd::dual_mark_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(*g, (uint4 *)fwd_pack_dev, (const uint4 *)rev_pack_dev);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CS_OK : dcuda(e, "dual_pack_kernel launch");
 }
@@ -2040,9 +2118,9 @@ cs_status cs_plan_dual(const cs_dual_graph *g, int32_t mode, int32_t k, int32_t 
     if (sms <= 0) return dfail(CS_ERR_CUDA, "no CUDA device");
     int bpsm = 0;
     const int mb = dual_minb();
-    cudaError_t e = mb == 4   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<4>, 256, 0)
-                    : mb == 3 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<3>, 256, 0)
-                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<2>, 256, 0);
+    cudaError_t e = mb == 4   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<4, csd::DPM>, 256, 0)
+                    : mb == 3 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<3, csd::DPM>, 256, 0)
+                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, csd::dual_kernel<2, csd::DPM>, 256, 0);
     if (e != cudaSuccess) return dcuda(e, "occupancy query");
     int slots = sms * std::max(1, bpsm) * 8;
     if (max_slots > 0) slots = std::min(slots, max_slots);

@@ -123,3 +123,18 @@ def test_simplest_capacity_chain_and_replay_counts():
             else:
                 assert_close_sums(got[m, i][idx], getattr(want, name)[dist], rtol=1e-9, atol=1e-9,
                                   what=f"{name}[{dist}] (cap 64)")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spokes", [5, 6, 7])
+def test_streets_with_many_edges_at_one_end(spokes):
+    """A hub of 5 streets gives each of them 4 dual edges at that end, the most of the narrow kernel; 6
+    and 7 take the wide one.  A ring joins the spokes' outer ends (2 more streets there)."""
+    ang = 2 * np.pi * np.arange(spokes) / spokes + 0.05 * np.arange(spokes)
+    r = 100.0 + 7.0 * np.arange(spokes)
+    x, y = np.r_[0.0, r * np.cos(ang)], np.r_[0.0, r * np.sin(ang)]
+    ring = np.arange(1, spokes)
+    u, v = np.r_[np.zeros(spokes, np.int64), ring], np.r_[np.arange(1, spokes + 1), ring + 1]
+    p = synth.Primal(x=x, y=y, u=u, v=v, length=np.hypot(x[v] - x[u], y[v] - y[u]).astype(np.float32),
+                     angle_sum=np.zeros(len(u), np.float32), geoms=[None] * len(u))
+    _run(synth.dual_structure(p), [150, 400])
