@@ -30,6 +30,7 @@
 #include <cmath>
 
 #include "cs_common.cuh"
+#include "cs_seed.cuh"
 #include "cs_sort.cuh"
 
 extern "C" void cs_set_error_internal(const char *msg);
@@ -1008,11 +1009,6 @@ __device__ int dual_replay(const DualParams &p, const DSlot &s, int src, int R, 
 // ------------------------------------------------------------------------------------------
 // D + E. Node best, closeness, backward sweep.
 // ------------------------------------------------------------------------------------------
-// Comparisons of the f64 values here (>= 0, finite) by their bits: no use of the f64 pipe, which GB300
-// runs at 1/64 of the f32 rate.
-__device__ __forceinline__ bool is_zero(double x) { return __double_as_longlong(x) == 0ll; }
-__device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
-
 template <int W>
 __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, int R, int *cnt, bool &bad, long long *ph) {
     long long tph = clock64();
@@ -1074,7 +1070,7 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
         for (int q = 0; q < K; q++) dl[(size_t)i * K + q] = 0.0;
     __syncwarp();
     const bool unit_wt = (wt == 1.0f);
-    const double wtd = (double)wt;
+    const double wtd = f2d(wt);
     const float one_tol = 1.0f + p.tol;
     const int nchunks = (R + 31) / 32;
     for (int ch = nchunks - 1; ch >= 0; ch--) {

@@ -620,9 +620,15 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
             const bool ready = !mine && ((blk & ~done) == 0u);
             if (ready) {
                 double sg = (i == 0) ? 1.0 : 0.0;
+                const unsigned rest = pm & (pm - 1u);
 #pragma unroll
                 for (int j = 0; j < PM; j++)
-                    if ((pm >> j) & 1u) sg = __dadd_rn(sg, sig[nb.pos[j]]);
+                    if (((pm & ~rest) >> j) & 1u) sg = sig[nb.pos[j]];  // the first predecessor: nothing to add to
+                if (rest) {
+#pragma unroll
+                    for (int j = 0; j < PM; j++)
+                        if ((rest >> j) & 1u) sg = __dadd_rn(sg, sig[nb.pos[j]]);
+                }
                 sig[i] = sg;
                 const int li0 = lane_index(i, K, nk, cum);
                 for (int k = first_k(p, route_cost(s.sd[i], p.speed)); k < K; k++) {
@@ -696,10 +702,12 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
     // --- backward Brandes sweep, all K thresholds in one pass (rust/src/centrality.rs:823-873,
     // 1782-1835), in the reference's f64: path counts, predecessor factors sigma_v / sigma_w, seeds
     // (pair count, and pair count * exp(-beta * cost) with the product and exp in f64) and
-    // dependencies.
+    // dependencies.  GB300 runs f64 at 1/64 of the f32 rate, so f64 instructions are spent on sums and shares
+    // alone: comparisons go by the bits, the seed's double-float is put together in integers, and what a
+    // node received is its credit as it is.
     __syncwarp();
     const bool unit_wt = (wt == 1.0f);
-    const double wtd = (double)wt;
+    const double wtd = f2d(wt);
     const int nchunks = failed ? 0 : (Rb + 31) / 32;
     constexpr int BW = (PM < BW_COLS) ? PM : BW_COLS;  // predecessors kept in this lane's shared column
     for (int ch = nchunks - 1; ch >= 0; ch--) {
@@ -733,18 +741,21 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
                     if (r < np) {
                         const double sv = sig[pl[r]];
                         bw_pl[r * 32 + lane] = lane_index(pl[r], K, nk, cum);
-                        bw_fr[r * 32 + lane] = (sv == sw) ? 1.0 : __ddiv_rn(sv, sw);
+                        bw_fr[r * 32 + lane] = same_bits(sv, sw) ? 1.0 : __ddiv_rn(sv, sw);
                     }
                 }
                 double *dli = dl + lane_index(i, K, nk, cum);
                 const int k0 = first_k(p, cost);
                 for (int k = k0; k < K; k++) {
-                    if (sw == 0.0) break;
-                    const double seed = (i == 0) ? 0.0 : pair;
-                    const double seedb = (i == 0 || pairf == 0.0f) ? 0.0 : seed_exp(pairf, p.beta[k], cost);
-                    const double dep = __dadd_rn(seed, __ldcg(&dli[2 * k]));
-                    const double depb = __dadd_rn(seedb, __ldcg(&dli[2 * k + 1]));
-                    if (dep == 0.0 && depb == 0.0) continue;
+                    if (is_zero(sw)) break;
+                    const double credit = __ldcg(&dli[2 * k]), creditb = __ldcg(&dli[2 * k + 1]);
+                    double dep = (i == 0) ? 0.0 : pair;
+                    double depb = (i == 0 || pairf == 0.0f) ? 0.0 : seed_exp(pairf, p.beta[k], cost);
+                    if (!is_zero(credit) || !is_zero(creditb)) {  // a leaf of the paths has its seed only
+                        dep = __dadd_rn(dep, credit);
+                        depb = __dadd_rn(depb, creditb);
+                    }
+                    if (is_zero(dep) && is_zero(depb)) continue;
 #pragma unroll 1
                     for (int r = 0; r < np; r++) {
                         int q;
@@ -755,21 +766,24 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
                         } else {  // beyond the shared column (high-degree graphs): from the scratch
                             const int qp = s.pr[(size_t)i * P + r];
                             const double sv = sig[qp];
-                            f = (sv == sw) ? 1.0 : __ddiv_rn(sv, sw);
+                            f = same_bits(sv, sw) ? 1.0 : __ddiv_rn(sv, sw);
                             q = lane_index(qp, K, nk, cum);
                         }
-                        if (f == 0.0) continue;
+                        if (is_zero(f)) continue;
                         double *pd = dl + q;
-                        atomicAdd(&pd[2 * k], f == 1.0 ? dep : __dmul_rn(f, dep));
-                        atomicAdd(&pd[2 * k + 1], f == 1.0 ? depb : __dmul_rn(f, depb));
+                        double f0 = dep, f1 = depb;
+                        if (!same_bits(f, 1.0)) {
+                            f0 = __dmul_rn(f, f0);
+                            f1 = __dmul_rn(f, f1);
+                        }
+                        atomicAdd(&pd[2 * k], f0);
+                        atomicAdd(&pd[2 * k + 1], f1);
                     }
                     if (v == src) continue;
-                    const double credit = __dadd_rn(dep, -seed);
-                    const double creditb = __dadd_rn(depb, -seedb);
                     constexpr size_t row_b = OD ? 0 : 5;
-                    if (credit > 0.0)
+                    if (__double_as_longlong(credit) > 0ll)
                         atomicAdd(p.out + (row_b * K + k) * N + v, unit_wt ? credit : __dmul_rn(credit, wtd));
-                    if (creditb > 0.0)
+                    if (__double_as_longlong(creditb) > 0ll)
                         atomicAdd(p.out + ((row_b + 1) * K + k) * N + v, unit_wt ? creditb : __dmul_rn(creditb, wtd));
                 }
                 mine = true;

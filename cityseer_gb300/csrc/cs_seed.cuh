@@ -83,6 +83,23 @@ __device__ __forceinline__ bool seed_exp_df(float beta, float cost, dfloat &r) {
     return true;
 }
 
+// h + l of a normalised double-float pair (|l| <= ulp(h) / 2, h normal) as f64, by integer arithmetic on
+// the f64's bits: l in units of its last place.
+__device__ __forceinline__ double df_to_d(dfloat r) {
+    const uint32_t b = __float_as_uint(r.h);
+    const int e = (int)((b >> 23) & 0xffu);
+    if (e < 56 || e > 202) return f2d(r.h) + f2d(r.l);
+    // below a power of two the f64's last place is half as large
+    const int q = 52 + ((b & 0x7fffffu) == 0u && r.l < 0.0f ? 1 : 0);
+    const float scale = __uint_as_float((uint32_t)(127 + q - (e - 127)) << 23);
+    const long long n = (long long)__float2int_rn(fmul(r.l, scale));
+    return __longlong_as_double(__double_as_longlong(f2d(r.h)) + n);
+}
+
+// Comparisons of f64 values >= 0 by their bits, without the f64 pipe.
+__device__ __forceinline__ bool is_zero(double x) { return __double_as_longlong(x) == 0ll; }
+__device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
+
 // w * exp(-(beta * cost)) as f64, for a pair weight w (0.5 or 1 for centrality, a trip weight for
 // origin-destination betweenness); the product with w is taken in double-float.
 __device__ __forceinline__ double seed_exp(float w, float beta, float cost) {
@@ -91,8 +108,13 @@ __device__ __forceinline__ double seed_exp(float w, float beta, float cost) {
         const dfloat y = df_two_prod(beta, cost);
         return (double)w * exp(-((double)y.h + (double)y.l));
     }
-    if (w != 1.0f) r = df_mul(r, {w, 0.0f});
-    return f2d(r.h) + f2d(r.l);
+    if (w == 0.5f) {
+        r.h = __fmul_rn(r.h, 0.5f);
+        r.l = __fmul_rn(r.l, 0.5f);
+    } else if (w != 1.0f) {
+        r = df_mul(r, {w, 0.0f});
+    }
+    return df_to_d(r);
 }
 
 }  // namespace cs

@@ -252,32 +252,6 @@ __device__ __forceinline__ double slow_sum(double d) {
     return d;
 }
 
-// h + l of a normalised double-float pair (|l| <= ulp(h) / 2, h normal) as f64, by integer arithmetic on
-// the f64's bits: l in units of its last place.
-__device__ __forceinline__ double df_to_d(dfloat r) {
-    const uint32_t b = __float_as_uint(r.h);
-    const int e = (int)((b >> 23) & 0xffu);
-    if (e < 56 || e > 202) return f2d(r.h) + f2d(r.l);
-    // below a power of two the f64's last place is half as large
-    const int q = 52 + ((b & 0x7fffffu) == 0u && r.l < 0.0f ? 1 : 0);
-    const float scale = __uint_as_float((uint32_t)(127 + q - (e - 127)) << 23);
-    const long long n = (long long)__float2int_rn(fmul(r.l, scale));
-    return __longlong_as_double(__double_as_longlong(f2d(r.h)) + n);
-}
-
-// w * exp(-(beta * cost)) as seed_exp (cs_seed.cuh), without its f64 add.
-__device__ __forceinline__ double seed_term(float w, float beta, float cost) {
-    dfloat r;
-    if (!seed_exp_df(beta, cost, r)) return seed_exp(w, beta, cost);
-    if (w == 0.5f) {
-        r.h = fmul(r.h, 0.5f);
-        r.l = fmul(r.l, 0.5f);
-    } else if (w != 1.0f) {
-        r = df_mul(r, {w, 0.0f});
-    }
-    return df_to_d(r);
-}
-
 // ------------------------------------------------------------------------------------------
 // 1. The union of the reached sets, numbered; the tile's adjacency.
 // ------------------------------------------------------------------------------------------
@@ -1043,7 +1017,7 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
                     if (seeded) {
                         if constexpr (OD) dep = f2d(pairf);
                         else dep = __hiloint2double(pairf == 1.0f ? 0x3ff00000 : 0x3fe00000, 0);
-                        depb = seed_term(pairf, p.beta[k], cost);
+                        depb = seed_exp(pairf, p.beta[k], cost);
                     }
                     double *row = a.dep + (size_t)(dep0 + (k - kmin)) * 64 + lane;
                     // rows below a successor's first threshold do not exist: it is beyond k for every lane
