@@ -1431,9 +1431,12 @@ __global__ void __launch_bounds__(256, MINB) dual_sync_kernel(const DualParams p
     if (lane < 16) ph[lane] = 0;
     __syncwarp();
     long long relaxed = 0, settled = 0, done_src = 0;
+    // sources claimed at a time: a round of the block's warps, or fewer when the launch has fewer sources
+    // than warps, so that they spread over all blocks (and SMs) instead of filling the first
+    const int claim = max(0, min(nw, (int)min((p.n_src + gridDim.x - 1) / (long long)gridDim.x, 32ll)));
     while (true) {
         if (threadIdx.x == 0) {
-            blk_base = atomicAdd(p.pass ? &p.hdr->work_next2 : &p.hdr->work_next, (unsigned long long)max(nw, 0));
+            blk_base = atomicAdd(p.pass ? &p.hdr->work_next2 : &p.hdr->work_next, (unsigned long long)claim);
             blk_err = __ldcg(&p.hdr->err);
         }
         __syncthreads();
@@ -1442,7 +1445,7 @@ __global__ void __launch_bounds__(256, MINB) dual_sync_kernel(const DualParams p
         __syncthreads();
         if (nw <= 0 || b0 >= (unsigned long long)p.n_src || berr != 0u) break;
         const unsigned long long idx = b0 + wib;
-        const bool mine = has_slot && idx < (unsigned long long)p.n_src;
+        const bool mine = wib < claim && idx < (unsigned long long)p.n_src;
         const int li = mine ? (p.remap ? p.remap[idx] : (int)idx) : 0;
         const int src = mine ? p.src_list[li] : 0;
         if (run_dual_source_sync<W>(p, s, mine, li, src, hist_all[wib], cnt_all[wib], ph, relaxed, settled)) {

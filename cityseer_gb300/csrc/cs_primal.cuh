@@ -500,6 +500,12 @@ __device__ __forceinline__ int load_preds(const SlotPtrs &s, int i, int P, int *
     return np;
 }
 
+// Sources a block of nw warps claims at a time: a whole round of its warps, or fewer when the launch has
+// fewer sources than warps, so that they spread over all blocks (and SMs) instead of filling the first.
+__device__ __forceinline__ int block_claim(int nw, long long n) {
+    return max(0, min(nw, (int)min((n + gridDim.x - 1) / (long long)gridDim.x, 32ll)));
+}
+
 // Phase barrier of the block-synchronous forms: GW warps (a whole 8-warp block: __syncthreads;
 // 4: a named barrier per half block) meet at the end of each phase.  GW = 0: no barrier.
 template <int GW>
@@ -1316,9 +1322,10 @@ __global__ void __launch_bounds__(256, MINB) segment_sync_kernel(const PrimalPar
     long long *ph = ph_all[wib];
     if (lane < 8) ph[lane] = 0;
     __syncwarp();
+    const int claim = block_claim(nw, p.n_src);
     while (true) {
         if (threadIdx.x == 0) {
-            blk_base = atomicAdd(p.rerun ? &p.hdr->work_next2 : &p.hdr->work_next, (unsigned long long)max(nw, 0));
+            blk_base = atomicAdd(p.rerun ? &p.hdr->work_next2 : &p.hdr->work_next, (unsigned long long)claim);
             blk_err = __ldcg(&p.hdr->err);
         }
         __syncthreads();
@@ -1327,7 +1334,7 @@ __global__ void __launch_bounds__(256, MINB) segment_sync_kernel(const PrimalPar
         __syncthreads();
         if (nw <= 0 || b0 >= (unsigned long long)p.n_src || berr != 0u) break;
         const unsigned long long idx = b0 + wib;
-        const bool mine = has_slot && idx < (unsigned long long)p.n_src;
+        const bool mine = wib < claim && idx < (unsigned long long)p.n_src;
         const int li = mine ? (p.remap ? p.remap[idx] : (int)idx) : 0;
         const int src = mine ? p.src_list[li] : 0;
         if (run_segment_sync<PM>(p, s, mine, li, src, hist_all[wib], queue_all[wib], ph, relaxed, settled)) {
@@ -1400,10 +1407,11 @@ __global__ void __launch_bounds__(WPB * 32, MINB) primal_sync_kernel(const Prima
     if (lane < 8) ph[lane] = 0;
     __syncwarp();
     const long long n = p.n_src;
+    const int claim = block_claim(nw, n);  // one group per block (GW = WPB)
     while (true) {
         if (gw == 0 && lane == 0) {
             blk_base[grp] = (long long)atomicAdd(p.rerun ? &p.hdr->work_next2 : &p.hdr->work_next,
-                                                 (unsigned long long)max(nw, 0));
+                                                 (unsigned long long)claim);
             blk_err[grp] = __ldcg(&p.hdr->err);
         }
         phase_barrier<GW>();
@@ -1412,7 +1420,7 @@ __global__ void __launch_bounds__(WPB * 32, MINB) primal_sync_kernel(const Prima
         phase_barrier<GW>();
         if (nw <= 0 || base >= n || berr != 0u) break;
         const long long idx = base + gw;
-        const bool mine = has_slot && idx < n;
+        const bool mine = gw < claim && idx < n;
         const int li = mine ? (p.remap ? p.remap[idx] : (int)idx) : 0;
         const int src = mine ? p.src_list[li] : 0;
         long long t0 = clock64();
@@ -1583,9 +1591,10 @@ __global__ void __launch_bounds__(256, MINB) batch_sync_kernel(const PrimalParam
     __shared__ PrimalParams pj_all[8];  // the warps' job parameters (as in batch_kernel)
     PrimalParams &p = pj_all[wib];
     int cur_job = -1;
+    const int claim = block_claim(nw, n);
     while (true) {
         if (threadIdx.x == 0) {
-            blk_base = (long long)atomicAdd(&base.hdr->work_next, (unsigned long long)max(nw, 0));
+            blk_base = (long long)atomicAdd(&base.hdr->work_next, (unsigned long long)claim);
             blk_err = __ldcg(&base.hdr->err);
         }
         __syncthreads();
@@ -1594,7 +1603,7 @@ __global__ void __launch_bounds__(256, MINB) batch_sync_kernel(const PrimalParam
         __syncthreads();
         if (nw <= 0 || b0 >= n || berr != 0u) break;
         const long long idx = b0 + wib;
-        const bool mine = has_slot && idx < n;
+        const bool mine = wib < claim && idx < n;
         int src = 0, li = 0;
         const long long item = item_lo + idx;
         if (mine) {
