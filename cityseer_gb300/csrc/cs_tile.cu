@@ -16,7 +16,7 @@
 // Phases of one tile, the block's warps together:
 //  1. Union: a banded label-correcting search ("near-far" delta-stepping) from all sources at once
 //     gives each node its least distance over the sources.  Nodes are numbered as they are found, so
-//     numbers ascend with that distance up to about a street's length.  Then the tile's adjacency
+//     numbers ascend with that distance up to about a band's width.  Then the tile's adjacency
 //     (neighbour number, both directions' seconds, the neighbour's slot of the edge back).
 //  2. Search: nodes whose row may improve are bits in shared memory; each round takes the lowest
 //     numbered 64 of them, and a warp pulls min(row, neighbour row + seconds).  A node that improved
@@ -46,6 +46,8 @@
 //    target, and the next level's lines are prefetched: 205 ms.
 //  - Consecutive items to different warps: 182 ms (1.8 instructions per cycle; stalls: barriers, then
 //    loads).  Blocks of 512 threads, 2 per SM: 256 x 4 ran 200 ms, 384 x 2 211 ms, 1024 x 1 226 ms.
+//  - Cheaper seeds and f64 only for sums and shares: 175 ms.  A wider union band, the next node's line
+//    loaded while closeness sums the last: 172 ms.
 //  - 16 partly ready nodes per level give 10,608 items in 114 levels per tile; letting all of them go
 //    gave 13,317 items (+25% sweep), 4 per level 370 levels (+60% time).
 #include <algorithm>
@@ -59,6 +61,9 @@ namespace tile {
 
 constexpr int BATCH = 64;         // nodes of one search round
 constexpr int LIST = 256;         // candidates of one schedule step
+// The union search only orders and bounds the tile: wider bands than a search's (fewer rounds, each a
+// chain of loads and barriers) suit it; 2x and 4x took 2.2 and 3.0 of a city pass's 175 ms off.
+constexpr float UNION_BAND = 4.0f;
 constexpr int UNPAIRED_SLOT = 9;  // header word: the graph has an edge without one back
 constexpr int PART = 16;          // partly ready nodes that each step lets go
 constexpr int MAX_ROUNDS = 1 << 17;  // bounded loops (never reached on a consistent graph)
@@ -278,7 +283,8 @@ __device__ void discover(const Params &p, const Arrays &a, const Smem &sm, float
         }
     }
     __syncthreads();
-    float T = p.delta;
+    const float band = p.delta * UNION_BAND;
+    float T = band;
     int nnear = v.nnear;
     for (int round = 0; round < MAX_ROUNDS; round++) {
         if (nnear > 0) {
@@ -330,7 +336,7 @@ __device__ void discover(const Params &p, const Arrays &a, const Smem &sm, float
         const int nfar = v.nfar;
         if (nfar == 0) return;
         const float mn = __int_as_float(v.fmn);
-        T = fmaxf(fadd(mn, p.delta), __int_as_float(__float_as_int(mn) + 1));
+        T = fmaxf(fadd(mn, band), __int_as_float(__float_as_int(mn) + 1));
         __syncthreads();
         if (tid == 0) {
             v.fmn = INF_BITS;
@@ -901,9 +907,15 @@ __device__ void closeness(const Params &p, const Arrays &a, const Smem &sm) {
     const int my_loc = v.loc[lane];
     const float wt = on ? v.wt[lane] : 0.0f;
     const bool unit = __all_sync(FULL, !on || wt == 1.0f);
+    float d_next = w < R ? a.dist[(size_t)w * 32 + lane] : 0.0f;
+    uint4 n_next = w < R ? *(const uint4 *)&a.node[w] : make_uint4(0u, 0u, 0u, 0u);
     for (int i = w; i < R; i += NW) {
-        const float d = a.dist[(size_t)i * 32 + lane];
-        const Node nd = a.node[i];
+        const float d = d_next;
+        const Node nd{n_next.x, n_next.y, (int)n_next.z, 0u};
+        if (i + NW < R) {  // the next node's row while this one is summed
+            d_next = a.dist[(size_t)(i + NW) * 32 + lane];
+            n_next = *(const uint4 *)&a.node[i + NW];
+        }
         const int kmin = (nd.info >> 16) & 0xff;
         const int t = nd.id;
         const float c = fmul(d, p.speed);
