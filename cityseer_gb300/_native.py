@@ -21,6 +21,7 @@ CS_ERR_CUDA = 3
 CS_ERR_TIMEOUT = 4
 CS_ERR_INTERNAL = 5
 CS_BATCH_ASYNC = 1
+CS_BATCH_NEAR_SOURCES = 2
 
 _ptr = C.c_void_p
 

@@ -1,7 +1,8 @@
 """Batched persistent form: many graphs, thresholds and modes in one persistent launch.
 
 Every (job, source) pair is an item of one device queue that the warps of a single persistent
-launch (`batch_kernel`) drain.  Small and large graphs share the GPU, so there is no per-graph
+launch (`batch_kernel`) drain; shortest-path jobs of wide reach go through one tiled launch instead
+(`tile_batch_kernel`, 32 nearby sources per block).  Small and large graphs share the GPU, so there is no per-graph
 launch tail and no per-graph host synchronisation.  The whole enqueue (resets, launch, threshold
 prefixes) is CUDA-graph capturable: `Batch.capture()` records it once, `Batch.replay()` re-runs it.
 The schedule -- band width per job and the register budget -- comes from `autotune`.
@@ -115,7 +116,20 @@ class Batch:
             if j in used and self.jobs[j]["mode"] == 1:
                 continue
             table.append(st)
-        table.sort(key=lambda st: {0: 0, 1: 1, 3: 2}[st.mode])  # one launch per mode group
+        # one launch per mode group; shortest-path jobs by their reach against a tile of 32 sources, widest
+        # first, which is what the tiled launch takes jobs by
+        def tiles(st):
+            if st.mode != 0 or st.n_sources == 0 or st.delta_seconds <= 0:
+                return 0.0
+            return -max(st.seconds[:st.k]) / st.delta_seconds * (st.n_sources / max(1, st.g.n_bound)) ** 0.5
+
+        table.sort(key=lambda st: ({0: 0, 1: 1, 3: 2}[st.mode], tiles(st)))
+        self.flags = 0
+        if sum(st.n_sources for st in table if st.mode == 0) >= centrality.TILE_CALL:
+            self.flags = _native.CS_BATCH_NEAR_SOURCES
+            for jb in self.jobs:
+                if jb["mode"] == 0 and len(jb["proc"]):
+                    jb["keep"][0].copy_(torch.from_numpy(centrality.spatial_order(jb["ns"], jb["proc"], 0)))
         self.n_fused = sum(1 for jb in self.jobs if "fused_with" in jb)
         self.table = (_native.BatchJob * len(table))(*table)
         n = C.c_int64()
@@ -144,7 +158,7 @@ class Batch:
         """Enqueues the whole batch; outputs must be zero (fresh Batch, or zero_outputs())."""
         st = stream if stream is not None else torch.cuda.current_stream().cuda_stream
         rc = self.lib.cs_batch_run(self.table, self.table_dev.data_ptr(), len(self.table), C.byref(self.plan),
-                                   self.ws.ptr, self.ws.nbytes, _native.CS_BATCH_ASYNC if async_ else 0, st)
+                                   self.ws.ptr, self.ws.nbytes, self.flags | (_native.CS_BATCH_ASYNC if async_ else 0), st)
         if rc != _native.CS_OK:
             self.ws.init(st)
             for jb in self.jobs:

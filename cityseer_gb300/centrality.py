@@ -284,13 +284,13 @@ def _hilbert_rank(ns) -> np.ndarray:
 TILE_CALL = 8192  # no smaller call has a tile of 32 sources for every resident block
 
 
-def spatial_order(ns, process: np.ndarray) -> np.ndarray:
+def spatial_order(ns, process: np.ndarray, fewest: int = TILE_CALL) -> np.ndarray:
     """The sources of a large call reordered so that consecutive ones lie near one another: the tile
     kernel takes 32 consecutive sources per block, and their searches share what their reaches have in
     common (on the 202,500-node lattice at 5 km, rows of 32 nodes instead of compact groups cost it
-    2.3x).  Smaller calls keep their order."""
+    2.3x).  Calls of fewer sources than `fewest` keep their order."""
     process = np.ascontiguousarray(process, np.int32)
-    if len(process) < TILE_CALL:
+    if len(process) < fewest:
         return process
     at = _hilbert_rank(ns)[process]
     placed = np.full(ns.node_bound(), -1, np.int32)

@@ -301,14 +301,47 @@ bool block_schedule(long long n_src) {
 // 3.2 km at 100 m (32 hops), every node (19,600) 6.1 against 8.7, every second 4.4 against 5.0, every
 // fourth 4.1 against 3.2; 1.6 km (16 hops) 3.3 against 3.2; 500 m at 80 m 4.8 against 3.5.
 // CS_TILE=0 leaves every source to the other kernels, CS_TILE=1 takes every call the kernel can serve.
+long long tile_call() { return 32ll * cs::tile::BPSM * std::max(1, sm_count()); }
+bool tile_reach(long long n_src, int n_bound, float maxsec, float delta) {
+    if (!(delta > 0.0f)) return false;
+    const double hops = 2.0 * maxsec / delta, radius = std::sqrt(16.0 * n_bound / (double)n_src);
+    return hops >= 5.0 * radius;
+}
 // Returns the sources per tile, 0: not this kernel.
 int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float delta) {
     const char *e = getenv("CS_TILE");
     if (e && e[0] == '0') return 0;
     if (e && e[0] == '1') return (int)std::max(1ll, std::min(32ll, (n_src + blocks - 1) / blocks));
-    if (n_src < 32ll * cs::tile::BPSM * std::max(1, sm_count()) || !(delta > 0.0f)) return 0;
-    const double hops = 2.0 * maxsec / delta, radius = std::sqrt(16.0 * n_bound / (double)n_src);
-    return hops >= 5.0 * radius ? 32 : 0;
+    return n_src >= tile_call() && tile_reach(n_src, n_bound, maxsec, delta) ? 32 : 0;
+}
+
+// The shortest-path jobs of a batch that go to the tile kernel: the rule's reach for each job by itself, its
+// sources for all of them together (one launch serves them), where the caller vouches for the sources' order
+// (near: a tile of sources from all over a graph holds their whole reaches one by one).  They have to be
+// one run of consecutive jobs [lo, hi), and the list of sources left to the per-warp kernel has to hold all.
+// Measured on nine lattices of 2,500 to 22,200 nodes at 1.6 or 3.2 km, three with segments too: 52.5 ms a
+// replay against 57.4 (six of the nine jobs tiled).
+void tile_jobs(const cs_batch_job *jobs, int n_jobs, bool near, long long list, int &lo, int &hi) {
+    lo = hi = 0;
+    const char *e = getenv("CS_TILE");
+    if ((e && e[0] == '0') || (!near && !(e && e[0] == '1'))) return;
+    long long total = 0;
+    for (int j = 0; j < n_jobs; j++) {
+        const cs_batch_job &b = jobs[j];
+        if (b.mode != cs::MODE_SHORTEST || b.n_sources <= 0) continue;
+        uint32_t maxs = 0;
+        for (int i = 0; i < b.k; i++) maxs = std::max(maxs, b.seconds[i]);
+        if (!(b.delta_seconds > 0.0f)) continue;
+        if (!(e && e[0] == '1') && !tile_reach(b.n_sources, b.g.n_bound, (float)maxs, b.delta_seconds)) continue;
+        if (total == 0) lo = hi = j;
+        if (hi != j || total + b.n_sources > list) {
+            hi = lo;
+            return;
+        }
+        hi = j + 1;
+        total += b.n_sources;
+    }
+    if (!(e && e[0] == '1') && total < tile_call()) hi = lo;
 }
 
 // Settle-order sort: distance buckets by default, CS_SORT=radix selects the LSD radix sort.
@@ -376,6 +409,8 @@ cs_status reset_dense(char *dense, size_t stride, int n_bound, int n_slots, cuda
     return CS_OK;
 }
 
+constexpr int TILE_LEFT_SLOT = 10;  // header word: items that a batch's tiles left to the per-warp kernel
+
 // The tile kernel's view of a call.
 cs::tile::Params tile_params(const cs::PrimalParams &p, const Layout &lay, const cs::tile::Geometry &geo, int lanes) {
     cs::tile::Params c;
@@ -415,6 +450,7 @@ cs::tile::Params tile_params(const cs::PrimalParams &p, const Layout &lay, const
     c.reach = p.reach;
     c.hdr = p.hdr;
     c.failed = p.failed;
+    c.n_failed = &p.hdr->n_failed;
     c.fail_cap = p.fail_cap;
     c.dense = p.dense;
     c.dense_stride = p.dense_stride;
@@ -1052,6 +1088,20 @@ cs_status cs_batch_run(const cs_batch_job *jobs_host, const cs_batch_job *jobs_d
     cudaError_t e = cudaMemsetAsync(p.hdr, 0, sizeof(cs::WsHeader), stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch reset");
     if (n_items == 0) return CS_OK;
+    // jobs for the tile kernel
+    int t_lo = 0, t_hi = 0, t_k = 1;
+    cs::tile::Geometry geo{};
+    const int tile_blocks = std::max(1, std::min(sm_count() * cs::tile::BPSM, plan->n_slots));
+    if (P <= cs::tile::PMAX) tile_jobs(jobs_host, n_jobs, (flags & CS_BATCH_NEAR_SOURCES) != 0, lay.fail_cap, t_lo, t_hi);
+    for (int j = t_lo; j < t_hi; j++) {  // the layout that suits the job with the most dependency rows per node
+        float dk[cs::MAXK];
+        for (int i = 0; i < jobs_host[j].k; i++) dk[i] = (float)jobs_host[j].distances[i];
+        const cs::tile::Geometry g =
+            cs::tile::geometry((lay.compact_total / tile_blocks) & ~size_t(255), jobs_host[j].k, dk, false);
+        if (j == t_lo || g.mcap < geo.mcap) geo = g;
+        t_k = std::max(t_k, jobs_host[j].k);
+    }
+    if (geo.mcap < plan->cap) t_hi = t_lo;
     // consecutive jobs of one mode run as one launch of that mode's kernel (a smaller instruction
     // footprint than the all-mode kernel); more than four such runs use the all-mode kernel once
     struct Run {
@@ -1059,16 +1109,43 @@ cs_status cs_batch_run(const cs_batch_job *jobs_host, const cs_batch_job *jobs_d
         int mode;
     };
     std::vector<Run> runs;
-    for (int j = 0; j < n_jobs; j++) {
-        const int m = (jobs_host[j].mode == cs::MODE_SHORTEST || jobs_host[j].mode == cs::MODE_SEGMENT)
-                          ? jobs_host[j].mode : -1;
-        const long long lo = jobs_host[j].item_begin, hi = lo + std::max(0, jobs_host[j].n_sources);
-        if (!runs.empty() && runs.back().mode == m) runs.back().hi = hi;
-        else runs.push_back({lo, hi, m});
+    for (bool again = true; again;) {
+        again = false;
+        runs.clear();
+        for (int j = 0; j < n_jobs; j++) {
+            if (j >= t_lo && j < t_hi) continue;
+            const int m = (jobs_host[j].mode == cs::MODE_SHORTEST || jobs_host[j].mode == cs::MODE_SEGMENT)
+                              ? jobs_host[j].mode : -1;
+            const long long lo = jobs_host[j].item_begin, hi = lo + std::max(0, jobs_host[j].n_sources);
+            if (!runs.empty() && runs.back().mode == m && runs.back().hi == lo) runs.back().hi = hi;
+            else runs.push_back({lo, hi, m});
+        }
+        if (runs.size() > 4 && t_hi > t_lo) {
+            t_hi = t_lo;  // then without the tile kernel
+            again = true;
+        }
     }
     if (runs.size() > 4) runs.assign(1, Run{0, n_items, -1});
     st = launch_seed_table(stream, cs::launch_seed_table_batch);
     if (st != CS_OK) return st;
+    if (t_hi > t_lo) {
+        // The tile kernel, then the per-warp kernel over the items that it lists.  How many there are stays on
+        // the device, so that a captured batch needs no host in between; what overflows there is listed as
+        // ever, in the other list.
+        cs::tile::Params c = tile_params(p, lay, geo, 32);
+        c.failed = (int32_t *)(base + lay.failed2_off);
+        c.n_failed = (unsigned *)&p.hdr->pad[TILE_LEFT_SLOT];
+        e = cs::tile::launch_seed_table(stream);
+        if (e == cudaSuccess) e = cs::tile::launch_batch(c, jobs_dev, t_lo, t_hi, t_k, tile_blocks, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "tile_batch_kernel launch");
+        g_counters[3] += 2;
+        cs::PrimalParams p2 = p;
+        p2.rerun = 1;
+        p2.remap = c.failed;
+        p2.n_remap = c.n_failed;
+        st = launch_batch(p2, plan, jobs_dev, n_jobs, 0, n_items, plan->n_slots, cs::MODE_SHORTEST, stream);
+        if (st != CS_OK) return st;
+    }
     for (const Run &r : runs) {
         if (r.hi <= r.lo) continue;
         e = cudaMemsetAsync(&p.hdr->work_next, 0, sizeof(unsigned long long), stream);

@@ -129,6 +129,7 @@ struct PrimalParams {
     int32_t n_slots;
     int32_t rerun;
     const int32_t *remap;  // rerun: indices into src_list of the sources to redo
+    const unsigned *n_remap;  // batched rerun: how many there are, where the host has not read it (else n_src)
     int32_t mode;
     int32_t row_cap;
     int32_t *t_count, *t_node, *t_pred;
@@ -1539,11 +1540,11 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const PrimalParams bas
     PrimalParams &p = pj_all[wib];
     __syncwarp();
     int cur_job = -1;
+    const long long n = !base.rerun ? item_hi - item_lo : (base.n_remap ? (long long)*base.n_remap : base.n_src);
     while (true) {
         unsigned long long idx = 0;
         if (lane == 0) idx = atomicAdd(base.rerun ? &base.hdr->work_next2 : &base.hdr->work_next, 1ull);
         idx = __shfl_sync(FULL, idx, 0);
-        const long long n = base.rerun ? base.n_src : item_hi - item_lo;
         if ((long long)idx >= n) break;
         if (__ldcg(&base.hdr->err) != 0u) break;
         const long long item = base.remap ? (long long)base.remap[idx] : item_lo + (long long)idx;

@@ -1115,117 +1115,207 @@ __device__ void trips(const Params &p, const Arrays &a, const Smem &sm, const ui
     __syncthreads();
 }
 
+// What a block counts over its tiles, added to the header at its end.
+struct Counts {
+    unsigned long long done = 0;
+    long long ph[7] = {0, 0, 0, 0, 0, 0, 0};  // cycles: union, adjacency, search, replay, schedule, closeness, betweenness
+};
+
+// One tile: sources [base, base + nl) of p.src_list.  v.fail on entry: list them at once.
+template <bool OD>
+__device__ void run_tile(const Params &p, const Arrays &a, const Smem &sm, float *d1, uint32_t *aux, long long base,
+                         int nl, Counts &n) {
+    Vars &v = sm.v;
+    const int tid = threadIdx.x;
+    long long t0 = clock64();
+    auto mark_phase = [&](int q) {
+        const long long now = clock64();
+        n.ph[q] += now - t0;
+        t0 = now;
+    };
+    if (tid < 32) {
+        const int s = tid < nl ? __ldg(&p.src_list[base + tid]) : 0;
+        v.src[tid] = s;
+        v.loc[tid] = -1;
+        v.wt[tid] = (tid < nl && !OD) ? __ldg(&p.src_wt[s]) : 1.0f;
+        if (tid == 0) {
+            v.nl = nl;
+            v.ok = nl == 32 ? FULL : (1u << nl) - 1u;
+            v.tcount = 0u;
+        }
+    }
+    for (int i = tid; i < 2 * 32 * p.k; i += TPB) ((int *)sm.cnt)[i] = 0;
+    __syncthreads();
+    bool whole = false;  // the numbering lost nodes: reset the whole dense state
+    const bool skip = v.fail != 0;
+    __syncthreads();
+    if (!skip) {
+        discover(p, a, sm, d1, aux);
+        mark_phase(0);
+        whole = v.fail != 0;
+        __syncthreads();
+        if (!whole) {
+            if (tid < nl) v.loc[tid] = (int)aux[v.src[tid]] - 1;
+            __syncthreads();
+            adjacency(p, a, sm, d1, aux);
+        }
+    }
+    mark_phase(1);
+    if (!v.fail) search(p, a, sm);
+    mark_phase(2);
+    if (!v.fail) {
+        replay(p, a, sm);
+        mark_phase(3);
+        if (p.betweenness) {
+            links(p, a, sm);
+            schedule(p, a, sm);
+        }
+        mark_phase(4);
+    }
+    __syncthreads();
+    const bool fail = v.fail != 0;
+    const unsigned ok = fail ? 0u : v.ok;
+    if (tid < nl && !((ok >> tid) & 1u)) {
+        // nothing was written for this source: the per-warp kernel redoes it
+        const unsigned f = atomicAdd(p.n_failed, 1u);
+        if (f < (unsigned)p.fail_cap) p.failed[f] = (int)(p.item0 + base + tid);
+        else raise_err(p.hdr, CS_ERR_CAPACITY, 50);
+    }
+    if (ok) {
+        if (!OD && p.closeness) closeness(p, a, sm);
+        mark_phase(5);
+        if (p.betweenness) {
+            if (OD) trips(p, a, sm, aux);
+            backward<OD>(p, a, sm);
+        }
+        mark_phase(6);
+        n.done += __popc(ok);
+        if (tid == 0) atomicAdd(&p.hdr->pad[PROGRESS_SLOT], (unsigned long long)__popc(ok));
+    }
+    __syncthreads();
+    if (whole) {
+        for (int i = tid; i < p.n_bound; i += TPB) {
+            d1[i] = inf_f();
+            aux[i] = 0u;
+        }
+    } else if (!skip) {
+        const int R = v.R;
+        for (int i = tid; i < R; i += TPB) {
+            const int x = a.rl[i];
+            d1[x] = inf_f();
+            aux[x] = 0u;
+        }
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void flush_counts(WsHeader *h, const Vars &v, const Counts &n) {
+    if (threadIdx.x != 0) return;
+    atomicAdd(&h->edges_relaxed, v.relaxed);
+    atomicAdd(&h->nodes_settled, v.settled);
+    atomicAdd(&h->sources_done, n.done);
+    for (int q = 0; q < 7; q++) atomicAdd(&h->pad[q], (unsigned long long)n.ph[q]);
+}
+
 template <bool OD>
 __global__ void __launch_bounds__(TPB, BPSM) tile_kernel(const __grid_constant__ Params p) {
     extern __shared__ __align__(16) char sm_raw[];
     const Smem sm = smem(sm_raw, p.k, p.geo.mcap);
     Vars &v = sm.v;
-    const int tid = threadIdx.x;
     const Arrays a = arrays(p);
     float *d1 = (float *)(p.dense + p.dense_stride * (size_t)blockIdx.x);
     uint32_t *aux = (uint32_t *)(p.dense + p.dense_stride * (size_t)blockIdx.x + p.aux_off);
-    long long ph[7] = {0, 0, 0, 0, 0, 0, 0};
-    long long t0 = 0;
-    auto mark_phase = [&](int q) {
-        const long long now = clock64();
-        ph[q] += now - t0;
-        t0 = now;
-    };
-    if (tid == 0) v.settled = v.relaxed = 0ull;
-    unsigned long long done_src = 0;
+    Counts n;
+    if (threadIdx.x == 0) v.settled = v.relaxed = 0ull;
     while (true) {
-        if (tid == 0) {
+        if (threadIdx.x == 0) {
             v.base = (long long)atomicAdd(&p.hdr->work_next, 1ull) * p.lanes;
             v.herr = __ldcg(&p.hdr->err);
             v.fail = __ldcg(&p.hdr->pad[UNPAIRED_SLOT]) != 0ull;  // then no tile can be served here
-            v.tcount = 0u;
         }
         __syncthreads();
         const long long base = v.base;
         if (base >= p.n_src || v.herr != 0u) break;
-        const int nl = (int)min((long long)p.lanes, p.n_src - base);
-        if (tid < 32) {
-            const int s = tid < nl ? __ldg(&p.src_list[base + tid]) : 0;
-            v.src[tid] = s;
-            v.loc[tid] = -1;
-            v.wt[tid] = (tid < nl && !OD) ? __ldg(&p.src_wt[s]) : 1.0f;
-            if (tid == 0) {
-                v.nl = nl;
-                v.ok = nl == 32 ? FULL : (1u << nl) - 1u;
-            }
-        }
-        for (int i = tid; i < 2 * 32 * p.k; i += TPB) ((int *)sm.cnt)[i] = 0;
-        t0 = clock64();
-        __syncthreads();
-        bool whole = false;  // the numbering lost nodes: reset the whole dense state
-        const bool skip = v.fail != 0;
-        __syncthreads();
-        if (!skip) {
-            discover(p, a, sm, d1, aux);
-            mark_phase(0);
-            whole = v.fail != 0;
-            __syncthreads();
-            if (!whole) {
-                if (tid < nl) v.loc[tid] = (int)aux[v.src[tid]] - 1;
-                __syncthreads();
-                adjacency(p, a, sm, d1, aux);
-            }
-        }
-        mark_phase(1);
-        if (!v.fail) search(p, a, sm);
-        mark_phase(2);
-        if (!v.fail) {
-            replay(p, a, sm);
-            mark_phase(3);
-            if (p.betweenness) {
-                links(p, a, sm);
-                schedule(p, a, sm);
-            }
-            mark_phase(4);
-        }
-        __syncthreads();
-        const bool fail = v.fail != 0;
-        const unsigned ok = fail ? 0u : v.ok;
-        if (tid < nl && !((ok >> tid) & 1u)) {
-            // nothing was written for this source: the per-warp kernel redoes it
-            const unsigned f = atomicAdd(&p.hdr->n_failed, 1u);
-            if (f < (unsigned)p.fail_cap) p.failed[f] = (int)(base + tid);
-            else raise_err(p.hdr, CS_ERR_CAPACITY, 50);
-        }
-        if (ok) {
-            if (!OD && p.closeness) closeness(p, a, sm);
-            mark_phase(5);
-            if (p.betweenness) {
-                if (OD) trips(p, a, sm, aux);
-                backward<OD>(p, a, sm);
-            }
-            mark_phase(6);
-            done_src += __popc(ok);
-            if (tid == 0) atomicAdd(&p.hdr->pad[PROGRESS_SLOT], (unsigned long long)__popc(ok));
-        }
-        __syncthreads();
-        if (whole) {
-            for (int i = tid; i < p.n_bound; i += TPB) {
-                d1[i] = inf_f();
-                aux[i] = 0u;
-            }
-        } else if (!skip) {
-            const int R = v.R;
-            for (int i = tid; i < R; i += TPB) {
-                const int n = a.rl[i];
-                d1[n] = inf_f();
-                aux[n] = 0u;
-            }
-        }
-        __syncthreads();
+        run_tile<OD>(p, a, sm, d1, aux, base, (int)min((long long)p.lanes, p.n_src - base), n);
     }
-    if (tid == 0) {
-        atomicAdd(&p.hdr->edges_relaxed, v.relaxed);
-        atomicAdd(&p.hdr->nodes_settled, v.settled);
-        atomicAdd(&p.hdr->sources_done, done_src);
-        // phase cycles, summed per block: union, adjacency, search, replay, schedule, closeness, betweenness
-        for (int q = 0; q < 7; q++) atomicAdd(&p.hdr->pad[q], (unsigned long long)ph[q]);
+    flush_counts(p.hdr, v, n);
+}
+
+// A batch's jobs [lo, hi), their sources in tiles of 32: block-wide parameters in shared memory, rewritten
+// when the block's job changes (the tiles come in job order).
+__global__ void __launch_bounds__(TPB, BPSM) tile_batch_kernel(const __grid_constant__ Params base,
+                                                               const cs_batch_job *jobs, int lo, int hi, int kmax) {
+    extern __shared__ __align__(16) char sm_raw[];
+    __shared__ Params p;
+    const Smem sm = smem(sm_raw, kmax, base.geo.mcap);
+    Vars &v = sm.v;
+    const Arrays a = arrays(base);
+    float *d1 = (float *)(base.dense + base.dense_stride * (size_t)blockIdx.x);
+    uint32_t *aux = (uint32_t *)(base.dense + base.dense_stride * (size_t)blockIdx.x + base.aux_off);
+    Counts n;
+    int cur = -1;                 // thread 0: the job p holds, and the tiles of the jobs before the next one
+    long long before = 0, first = 0;
+    if (threadIdx.x == 0) {
+        v.settled = v.relaxed = 0ull;
+        cur = lo - 1;
     }
+    while (true) {
+        if (threadIdx.x == 0) {
+            const long long t = (long long)atomicAdd(&base.hdr->work_next, 1ull);
+            v.herr = __ldcg(&base.hdr->err);
+            v.fail = __ldcg(&base.hdr->pad[UNPAIRED_SLOT]) != 0ull;
+            int j = cur;
+            while (j < hi && t >= before) {
+                j++;
+                first = before;
+                if (j < hi) before += (max(jobs[j].n_sources, 0) + 31) / 32;
+            }
+            if (j >= hi) {
+                v.base = -1;
+            } else {
+                if (j != cur) {
+                    const cs_batch_job &b = jobs[j];
+                    p = base;
+                    p.n_bound = b.g.n_bound;
+                    p.in_ptr = b.g.in_ptr_dev;
+                    p.in_nb = b.g.in_nb_dev;
+                    p.in_w = b.g.in_w_dev;
+                    p.out_ptr = b.g.out_ptr_dev;
+                    p.out_to = b.g.out_to_dev;
+                    p.out_w = b.g.out_w_dev;
+                    p.out_cnt = b.g.out_cnt_dev;
+                    p.node_w = b.g.node_w_dev;
+                    p.k = b.k;
+                    uint32_t maxs = 0;
+                    for (int i = 0; i < b.k; i++) {
+                        p.dk[i] = (float)b.distances[i];
+                        p.beta[i] = b.betas[i];
+                        maxs = max(maxs, b.seconds[i]);
+                    }
+                    p.maxsec = (float)maxs;
+                    p.speed = b.speed_m_s;
+                    p.tol = b.tolerance;
+                    p.delta = b.delta_seconds;
+                    p.closeness = b.compute_closeness;
+                    p.betweenness = b.compute_betweenness;
+                    p.src_list = b.sources_dev;
+                    p.n_src = b.n_sources;
+                    p.src_wt = b.src_wt_dev;
+                    p.eligible = b.eligible_dev;
+                    p.out = b.out_dev;
+                    p.bucket = b.bucket_dev;
+                    p.item0 = b.item_begin;
+                    cur = j;
+                }
+                v.base = (t - first) * 32;
+            }
+        }
+        __syncthreads();
+        const long long at = v.base;
+        if (at < 0 || v.herr != 0u) break;
+        run_tile<false>(p, a, sm, d1, aux, at, (int)min(32ll, p.n_src - at), n);
+    }
+    flush_counts(base.hdr, v, n);
 }
 
 // ==========================================================================================
@@ -1281,6 +1371,15 @@ cudaError_t launch_t(const Params &p, int blocks, cudaStream_t stream) {
 
 cudaError_t launch(const Params &p, bool od, int blocks, cudaStream_t stream) {
     return od ? launch_t<true>(p, blocks, stream) : launch_t<false>(p, blocks, stream);
+}
+
+cudaError_t launch_batch(const Params &p, const cs_batch_job *jobs_dev, int lo, int hi, int kmax, int blocks,
+                         cudaStream_t stream) {
+    const size_t bytes = smem_bytes(kmax, p.geo.mcap);
+    const cudaError_t e = cudaFuncSetAttribute(tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    tile_batch_kernel<<<blocks, TPB, bytes, stream>>>(p, jobs_dev, lo, hi, kmax);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_seed_table(cudaStream_t stream) {

@@ -53,8 +53,10 @@ struct Params {
     uint32_t *reach;
     // workspace: the per-warp slots' clean dense arrays (block b uses slot b's) and their compact region
     WsHeader *hdr;
-    int32_t *failed;  // sources (indices into src_list) left to the per-warp kernel
+    int32_t *failed;  // item0 + the indices into src_list of the sources left to the per-warp kernel
+    unsigned *n_failed;
     int32_t fail_cap;
+    int64_t item0;
     char *dense;
     size_t dense_stride, aux_off;
     char *region;
@@ -65,6 +67,10 @@ struct Params {
 Geometry geometry(size_t region_bytes, int k, const float *dk, bool od);
 // Launches `blocks` persistent blocks on `stream`; returns the launch error.
 cudaError_t launch(const Params &p, bool od, int blocks, cudaStream_t stream);
+// Launches `blocks` persistent blocks over a batch's shortest-path jobs [lo, hi), at most kmax thresholds
+// each; p holds what the jobs share (scratch, header, lists).
+cudaError_t launch_batch(const Params &p, const cs_batch_job *jobs_dev, int lo, int hi, int kmax, int blocks,
+                         cudaStream_t stream);
 // Tabulates the seed exponentials of this kernel (cs_seed.cuh) on `stream`.
 cudaError_t launch_seed_table(cudaStream_t stream);
 

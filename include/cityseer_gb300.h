@@ -326,6 +326,10 @@ cs_status cs_tree_simplest(const cs_dual_graph *g, int32_t n_queries, const int3
  * as a batch without CS_BATCH_ASYNC).  Without the flag, overflowed items are redone inside the
  * call at growing capacities. */
 #define CS_BATCH_ASYNC 1
+/* cs_batch_run: consecutive entries of every shortest-path job's sources_dev lie near one another (on a
+ * space-filling curve, say), so that 32 of them can share a search.  Jobs of wide reach that are
+ * consecutive in the table then run through one tiled launch. */
+#define CS_BATCH_NEAR_SOURCES 2
 cs_status cs_batch_prepare(cs_batch_job *jobs_host, int32_t n_jobs, int64_t *n_items);
 cs_status cs_batch_plan(const cs_batch_job *jobs_host, int32_t n_jobs, int32_t cap, int32_t max_slots,
                         int64_t mem_budget_bytes, cs_plan *plan);

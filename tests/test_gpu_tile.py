@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from cityseer_gb300 import centrality, synth
+from cityseer_gb300.batch import Batch
 from cityseer_gb300.graph import NetworkStructure
 
 pytestmark = pytest.mark.gpu
@@ -130,6 +131,38 @@ def test_tile_weights_and_repeated_sources(tile):
             assert np.array_equal(np.isfinite(new), np.isfinite(col))
             ok = np.isfinite(col)  # a source of weight 0 has no cycles weight
             assert np.linalg.norm(new[ok] - col[ok]) <= 1e-10 * np.linalg.norm(col[ok])
+
+
+@pytest.mark.parametrize("graphs", [
+    ["plain", "diagonals"], ["two_nodes", "equal_distances", "plain"], ["exact_grid", "one_way", "parallel"],
+])
+def test_batched_tiles(tile, graphs):
+    """Jobs of one tiled launch, with another mode beside them; run at once and replayed from a capture."""
+    flags = [{}, dict(compute_betweenness=False), dict(compute_closeness=False)]
+    jobs = [dict(ns=GRAPHS[g](), mode="shortest", distances=[[300, 700, 1500], [900], [400, 1200]][i], **flags[i])
+            for i, g in enumerate(graphs)]
+    jobs.insert(1, dict(ns=jobs[0]["ns"], mode="segment", distances=[500]))
+    jobs.append(dict(ns=jobs[0]["ns"], mode="shortest", distances=[1100], source_indices=[0, 1]))
+    tile(False)
+    plain = Batch(jobs)
+    plain.run()
+    want = plain.results()
+    tile(True)
+    b = Batch(jobs)
+    b.run()
+    for got in (b.results(), None):
+        if got is None:
+            b.capture()
+            b.replay()
+            b.replay()
+            assert b.status()[0] == 0
+            got = b.results()
+        for g, w, j in zip(got, want, jobs):
+            if j["mode"] == "segment":
+                _compare(g, w, ("segment_density", "segment_betweenness"))
+            else:
+                _compare(g, w, [m for m in ROWS if (j.get("compute_closeness", True) or "between" in m)
+                                and (j.get("compute_betweenness", True) or "between" not in m)])
 
 
 @pytest.mark.parametrize("graph", ["diagonals", "exact_grid", "parallel"])
