@@ -165,6 +165,20 @@ def test_batched_tiles(tile, graphs):
                                 and (j.get("compute_betweenness", True) or "between" not in m)])
 
 
+def test_batched_tiles_beyond_one_list(tile):
+    ns = _lattice(300)  # three jobs of 90,000 sources: more than one launch's list of 2^18 holds
+    jobs = [dict(ns=ns, mode="shortest", distances=[d]) for d in (320, 240, 160)]
+    tile(False)
+    plain = Batch(jobs)
+    plain.run()
+    want = plain.results()
+    tile(True)
+    b = Batch(jobs)
+    b.run()
+    for g, w in zip(b.results(), want):
+        _compare(g, w, ROWS)
+
+
 @pytest.mark.parametrize("graph", ["diagonals", "exact_grid", "parallel"])
 def test_tile_trips(tile, graph):
     ns = GRAPHS[graph]()
