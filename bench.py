@@ -162,7 +162,12 @@ def cpu_baseline(ns, dists, n_total: int, target_seconds: float, nthreads: int |
     }
 
 
-def traffic_ratio(kernel: str = "primal_sync_kernel"):
+# cycle shares of the tile kernel's phases, and of the per-warp kernel's (smaller --side)
+TILE_PHASES = ("union", "adjacency", "search", "replay", "schedule", "closeness", "backward")
+WARP_PHASES = ("search", "sort", "replay", "closeness", "sigma", "backward", "reset")
+
+
+def traffic_ratio(kernel: str = "tile_kernel"):
     """DRAM bytes per algorithmic byte of the timed kernel, from the ncu figures kept in
     profiles/traffic.json (one capture of that kernel on a smaller lattice of the same recipe)."""
     try:
@@ -377,7 +382,7 @@ def run_gpu(args):
         "roofline": roofline,
         "gpu_launches": int(launches),
         "phase_share": {nm: round(v / max(1, sum(ph)), 4) for nm, v in
-                        zip(("search", "sort", "replay", "closeness", "sigma", "backward", "reset"), ph)},
+                        zip(TILE_PHASES if n_src >= centrality.TILE_CALL else WARP_PHASES, ph)},
         "clocks": clk,
     }
     if rank == 0 and ws == 1 and not args.no_cpu:  # the CPU baseline is reported at N = 1 only

@@ -74,10 +74,12 @@ typedef struct {
     const int32_t *rfrom_dev;   /* [n_edges] source node of each incoming edge */
     const int32_t *rid_dev;     /* [n_edges] index of that edge in the forward arrays */
     /* Packed 16-byte edge records (cs_dual_pack), required by the centrality calls (the tree calls
-     * read the plain arrays): fwd_pack [n_edges] in forward order = target state (2 to + entry_slot)
-     * | exit_slot << 31, then the f32 bits of w, angle_sum and length; rev_pack [n_edges] in reverse
-     * order = offering state (2 from + 1 - exit_slot) | entry_slot << 31, w, angle_sum, length.
-     * 16-byte aligned; n_bound < 2^30. */
+     * read the plain arrays): fwd_pack [n_edges] = target state (2 to + entry_slot) | exit_slot << 31,
+     * then the f32 bits of w, angle_sum and length; rev_pack [n_edges] = offering state
+     * (2 from + 1 - exit_slot) | entry_slot << 31, w, angle_sum, length.  Within a node the records are
+     * grouped by its own end (slot 0 first), else in forward / reverse order; the sign bit of the first
+     * forward record's w marks a graph with ends too wide for the common kernel.  16-byte aligned;
+     * n_bound < 2^30. */
     const void *fwd_pack_dev;
     const void *rev_pack_dev;
 } cs_dual_graph;
@@ -328,7 +330,7 @@ cs_status cs_tree_simplest(const cs_dual_graph *g, int32_t n_queries, const int3
 #define CS_BATCH_ASYNC 1
 /* cs_batch_run: consecutive entries of every shortest-path job's sources_dev lie near one another (on a
  * space-filling curve, say), so that 32 of them can share a search.  Jobs of wide reach that are
- * consecutive in the table then run through one tiled launch. */
+ * consecutive in the table then run as tiles (one launch for every 2^18 of their sources or more). */
 #define CS_BATCH_NEAR_SOURCES 2
 cs_status cs_batch_prepare(cs_batch_job *jobs_host, int32_t n_jobs, int64_t *n_items);
 cs_status cs_batch_plan(const cs_batch_job *jobs_host, int32_t n_jobs, int32_t cap, int32_t max_slots,
