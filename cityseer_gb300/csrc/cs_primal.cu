@@ -276,18 +276,24 @@ bool block_kernel_enabled() {
 }
 
 // Schedule of one call: one block per source gives a source a whole SM (the lowest latency per
-// source) and one warp per source keeps ~24 sources per SM in flight (the highest throughput).  Calls
-// with at most CS_BLOCK_SOURCES_MAX sources (default: 4 per SM) take the block kernel, larger ones
-// the per-warp kernel; CS_BLOCK_PER_SOURCE=1 forces the block kernel.  On the 202,500-node lattice
-// at 5 km a call of 8-152 sources took 1.2 ms with blocks and 5.0-5.3 ms with warps, 608 sources
-// 4.3 ms against 6.2 ms, and 1,216 sources 8.2 ms against 7.7 ms.
-bool block_schedule(long long n_src) {
+// source) and one warp per source keeps ~24 sources per SM in flight (the highest throughput).  Blocks
+// take the sources in waves of one per SM; a warp's time for one source hides all of them, and grows
+// faster with the reach than a block's.  So blocks pay for as many waves as the hops to the cutoff
+// (seconds / median edge seconds, half a plan's band width) over 13, between 1 and 5.  Measured, blocks
+// against warps (152 SMs, ms per call):
+//    6 hops   152 sources 0.433 / 0.461, 304 0.496 / 0.462     25 hops  304 1.020 / 1.087, 456 1.246 / 1.070
+//   12 hops   152 sources 0.510 / 0.592, 304 0.601 / 0.585     32 hops  304 1.129 / 1.445, 456 1.527 / 1.435
+//   16 hops   152 sources 0.442 / 0.559, 608 0.924 / 0.569     40 hops  456 1.947 / 2.185, 608 2.410 / 2.309
+//   62 hops   152 sources 1.442 / 4.643, 608 4.071 / 5.288, 700 4.874 / 5.315, 800 5.584 / 5.381
+// CS_BLOCK_SOURCES_MAX sets the most sources of a call for blocks; CS_BLOCK_PER_SOURCE=1 forces them.
+bool block_schedule(long long n_src, float maxsec, float delta) {
     const char *e = getenv("CS_BLOCK_PER_SOURCE");
     if (e && e[0] == '0') return false;
     if (e && e[0] == '1') return true;
     const char *m = getenv("CS_BLOCK_SOURCES_MAX");
-    const long long cap = m ? atoll(m) : 4ll * std::max(1, sm_count());
-    return n_src <= cap;
+    if (m) return n_src <= atoll(m);
+    const double waves = delta > 0.0f ? std::min(5.0, std::max(1.0, 2.0 * maxsec / delta / 13.0)) : 4.0;
+    return (double)n_src <= waves * std::max(1, sm_count());
 }
 
 // Tile kernel (cs_tile.cu): 32 nearby sources per block, one per lane.  A tile does its sources' common
@@ -495,8 +501,6 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
     if (plan->lanes < L) return fail(CS_ERR_ARG, "plan was made for fewer thresholds");
     if (plan->n_bound > 0 && plan->n_bound != g->n_bound)
         return fail(CS_ERR_ARG, "plan was made for a graph of another node bound");
-    const bool block = (mode == cs::MODE_SHORTEST || mode == cs::MODE_OD) && plan->cta_blocks > 0 &&
-                       cs::cta::supported(P, K) && q && block_schedule(q->n_sources);
     Layout lay = layout(g->n_bound, plan->n_slots, plan->cap, P, plan->lanes, plan->cta_blocks);
     if (ws_bytes < lay.total) return fail(CS_ERR_ARG, "workspace too small for this plan");
     cudaStream_t stream = (cudaStream_t)stream_v;
@@ -546,6 +550,8 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
     if (!(p.speed > 0.0f) || !std::isfinite(p.speed)) return fail(CS_ERR_ARG, "speed_m_s must be finite and positive");
     p.maxsec = (float)maxs;
     p.delta = plan->delta_seconds > 0.0f ? plan->delta_seconds : std::max(1.0f, p.maxsec / 48.0f);
+    const bool block = (mode == cs::MODE_SHORTEST || mode == cs::MODE_OD) && plan->cta_blocks > 0 &&
+                       cs::cta::supported(P, K) && q && block_schedule(q->n_sources, p.maxsec, plan->delta_seconds);
     p.out = out.out_dev;
     p.bucket = (double *)(base + lay.bucket_off);
     p.reach = out.reach_dev;

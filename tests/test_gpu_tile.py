@@ -133,6 +133,17 @@ def test_tile_weights_and_repeated_sources(tile):
             assert np.linalg.norm(new[ok] - col[ok]) <= 1e-10 * np.linalg.norm(col[ok])
 
 
+@pytest.mark.parametrize("distance,n_src", [(240, 1), (240, 152), (240, 153), (2800, 760), (2800, 761)])
+def test_blocks_or_warps_by_reach_and_count(monkeypatch, distance, n_src):
+    """One block per source or one warp per source, at the edges of the rule (few and many hops)."""
+    monkeypatch.setenv("CS_TILE", "0")
+    ns = _lattice(60)
+    src = [int(s) for s in np.random.default_rng(2).choice(3600, n_src, replace=False)]
+    by_rule = ns.centrality_shortest(distances=[distance], source_indices=src)
+    monkeypatch.setenv("CS_BLOCK_PER_SOURCE", "0")
+    _compare(by_rule, ns.centrality_shortest(distances=[distance], source_indices=src), ROWS)
+
+
 @pytest.mark.parametrize("graphs", [
     ["plain", "diagonals"], ["two_nodes", "equal_distances", "plain"], ["exact_grid", "one_way", "parallel"],
 ])
