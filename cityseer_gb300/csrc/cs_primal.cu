@@ -279,8 +279,9 @@ bool block_kernel_enabled() {
 // source) and one warp per source keeps ~24 sources per SM in flight (the highest throughput).  Blocks
 // take the sources in waves of one per SM; a warp's time for one source hides all of them, and grows
 // faster with the reach than a block's.  So blocks pay for as many waves as the hops to the cutoff
-// (seconds / median edge seconds, half a plan's band width) over 13, between 1 and 5.  Measured, blocks
-// against warps (152 SMs, ms per call):
+// (seconds / median edge seconds, half a plan's band width) over 13, between 1 and 4 (a fifth wave at
+// 5 km won 8% where every reach fitted a block's table, and lost more where some had to be redone by warps).
+// Measured, blocks against warps (152 SMs, ms per call):
 //    6 hops   152 sources 0.433 / 0.461, 304 0.496 / 0.462     25 hops  304 1.020 / 1.087, 456 1.246 / 1.070
 //   12 hops   152 sources 0.510 / 0.592, 304 0.601 / 0.585     32 hops  304 1.129 / 1.445, 456 1.527 / 1.435
 //   16 hops   152 sources 0.442 / 0.559, 608 0.924 / 0.569     40 hops  456 1.947 / 2.185, 608 2.410 / 2.309
@@ -292,7 +293,7 @@ bool block_schedule(long long n_src, float maxsec, float delta) {
     if (e && e[0] == '1') return true;
     const char *m = getenv("CS_BLOCK_SOURCES_MAX");
     if (m) return n_src <= atoll(m);
-    const double waves = delta > 0.0f ? std::min(5.0, std::max(1.0, 2.0 * maxsec / delta / 13.0)) : 4.0;
+    const double waves = delta > 0.0f ? std::min(4.0, std::max(1.0, 2.0 * maxsec / delta / 13.0)) : 4.0;
     return (double)n_src <= waves * std::max(1, sm_count());
 }
 

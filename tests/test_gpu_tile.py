@@ -133,7 +133,7 @@ def test_tile_weights_and_repeated_sources(tile):
             assert np.linalg.norm(new[ok] - col[ok]) <= 1e-10 * np.linalg.norm(col[ok])
 
 
-@pytest.mark.parametrize("distance,n_src", [(240, 1), (240, 152), (240, 153), (2800, 760), (2800, 761)])
+@pytest.mark.parametrize("distance,n_src", [(240, 1), (240, 152), (240, 153), (2800, 608), (2800, 609)])
 def test_blocks_or_warps_by_reach_and_count(monkeypatch, distance, n_src):
     """One block per source or one warp per source, at the edges of the rule (few and many hops)."""
     monkeypatch.setenv("CS_TILE", "0")
