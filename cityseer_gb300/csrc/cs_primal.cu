@@ -280,7 +280,7 @@ bool block_kernel_enabled() {
 // take the sources in waves of one per SM; a warp's time for one source hides all of them, and grows
 // faster with the reach than a block's.  So blocks pay for as many waves as the hops to the cutoff
 // (seconds / median edge seconds, half a plan's band width) over 13, between 1 and 4 (a fifth wave at
-// 5 km won 8% where every reach fitted a block's table, and lost more where some had to be redone by warps).
+// 5 km was 8% faster on one lattice, less than whole calls vary).
 // Measured, blocks against warps (152 SMs, ms per call):
 //    6 hops   152 sources 0.433 / 0.461, 304 0.496 / 0.462     25 hops  304 1.020 / 1.087, 456 1.246 / 1.070
 //   12 hops   152 sources 0.510 / 0.592, 304 0.601 / 0.585     32 hops  304 1.129 / 1.445, 456 1.527 / 1.435
