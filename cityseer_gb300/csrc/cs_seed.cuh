@@ -84,15 +84,17 @@ __device__ __forceinline__ bool seed_exp_df(float beta, float cost, dfloat &r) {
 }
 
 // h + l of a normalised double-float pair (|l| <= ulp(h) / 2, h normal) as f64, by integer arithmetic on
-// the f64's bits: l in units of its last place.
+// the f64's bits: l in units of its last place.  The bits hold a magnitude, so l counts towards it with
+// the sign it has against h's.
 __device__ __forceinline__ double df_to_d(dfloat r) {
     const uint32_t b = __float_as_uint(r.h);
     const int e = (int)((b >> 23) & 0xffu);
     if (e < 56 || e > 202) return f2d(r.h) + f2d(r.l);
+    const float l = __uint_as_float(__float_as_uint(r.l) ^ (b & 0x80000000u));
     // below a power of two the f64's last place is half as large
-    const int q = 52 + ((b & 0x7fffffu) == 0u && r.l < 0.0f ? 1 : 0);
+    const int q = 52 + ((b & 0x7fffffu) == 0u && l < 0.0f ? 1 : 0);
     const float scale = __uint_as_float((uint32_t)(127 + q - (e - 127)) << 23);
-    const long long n = (long long)__float2int_rn(fmul(r.l, scale));
+    const long long n = (long long)__float2int_rn(fmul(l, scale));
     return __longlong_as_double(__double_as_longlong(f2d(r.h)) + n);
 }
 
