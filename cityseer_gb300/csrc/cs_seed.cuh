@@ -101,6 +101,10 @@ __device__ __forceinline__ double df_to_d(dfloat r) {
 // Comparisons of f64 values >= 0 by their bits, without the f64 pipe.
 __device__ __forceinline__ bool is_zero(double x) { return __double_as_longlong(x) == 0ll; }
 __device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
+// x > 0.0 for any x: zero wraps round, NaN and negative values lie above the bits of infinity.
+__device__ __forceinline__ bool positive(double x) {
+    return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
+}
 
 // w * exp(-(beta * cost)) as f64, for a pair weight w (0.5 or 1 for centrality, a trip weight for
 // origin-destination betweenness); the product with w is taken in double-float.

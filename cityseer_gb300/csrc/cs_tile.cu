@@ -1073,15 +1073,17 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
                         row[0] = dep;
                         row[32] = depb;
                     }
-                    if (src || !on) acc = accb = 0.0;
+                    // a source credits a node only with what is positive, as the reference does per source
+                    if (src || !on || !positive(acc)) acc = 0.0;
+                    if (src || !on || !positive(accb)) accb = 0.0;
                     if (!unit) {
-                        acc = __dmul_rn(acc, f2d(wt));
-                        accb = __dmul_rn(accb, f2d(wt));
+                        if (!is_zero(acc)) acc = __dmul_rn(acc, f2d(wt));
+                        if (!is_zero(accb)) accb = __dmul_rn(accb, f2d(wt));
                     }
                     const FixSum s0 = fix_sum(acc), s1 = fix_sum(accb);
                     double val = fix_to_d(lane ? s1 : s0, 1081);
                     if ((s0.e < 64 && (s0.e < 0 || s0.sum)) || (s1.e < 64 && (s1.e < 0 || s1.sum))) {
-                        // not finite, negative, or close to the smallest f64
+                        // not finite, of a negative source weight, or close to the smallest f64
                         const double d0 = slow_sum(acc), d1 = slow_sum(accb);
                         val = lane ? d1 : d0;
                     }

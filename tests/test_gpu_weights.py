@@ -1,5 +1,5 @@
-"""Trip weights of either sign in the schedules of the shortest-path kernels: one warp per source and one
-block per source."""
+"""Trip weights of either sign, in each schedule of the shortest-path kernels: one warp per source, one
+block per source, and tiles of 32 sources (which calls of 10,000 sources of this reach take by themselves)."""
 import numpy as np
 import pytest
 import torch
@@ -11,7 +11,8 @@ from helpers import assert_close_sums
 
 pytestmark = pytest.mark.gpu
 
-SCHEDULES = {"warp": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "0"}, "block": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "1"}}
+SCHEDULES = {"warp": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "0"}, "block": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "1"},
+             "tile": {}}
 DISTANCES = [700, 2400]
 
 
