@@ -1141,7 +1141,7 @@ __device__ void dual_accumulate(const DualParams &p, const DSlot &s, int src, in
                     }
                     if (v == src) continue;
                     const double credit = __dadd_rn(dep, -seed);
-                    if (__double_as_longlong(credit) > 0ll)
+                    if (positive(credit))
                         atomicAdd(p.out + ((size_t)3 * K + k) * N + v, unit_wt ? credit : __dmul_rn(credit, wtd));
                 }
                 mine = true;

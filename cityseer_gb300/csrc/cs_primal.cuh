@@ -741,6 +741,8 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
                 if constexpr (OD) pairf = od_weight(p, src, v);
                 else pairf = __ldg(&p.eligible[v]) ? 0.5f : 1.0f;
                 const double pair = f2d(pairf);
+                // the reference's credit is dependency - seed: NaN, never positive, at a destination of such trips
+                const bool credited = !OD || fabsf(pairf) < __int_as_float(INF_BITS);
                 // predecessor rows and factors go to this lane's shared-memory column, so that the
                 // push loop below is a plain (not unrolled) loop over the np predecessors
 #pragma unroll
@@ -786,11 +788,11 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
                         atomicAdd(&pd[2 * k], f0);
                         atomicAdd(&pd[2 * k + 1], f1);
                     }
-                    if (v == src) continue;
+                    if (v == src || !credited) continue;
                     constexpr size_t row_b = OD ? 0 : 5;
-                    if (__double_as_longlong(credit) > 0ll)
+                    if (positive(credit))
                         atomicAdd(p.out + (row_b * K + k) * N + v, unit_wt ? credit : __dmul_rn(credit, wtd));
-                    if (__double_as_longlong(creditb) > 0ll)
+                    if (positive(creditb))
                         atomicAdd(p.out + ((row_b + 1) * K + k) * N + v, unit_wt ? creditb : __dmul_rn(creditb, wtd));
                 }
                 mine = true;
@@ -1049,8 +1051,8 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
                             if (isfinite(auc) && auc > 0.0f) total = __dadd_rn(total, f2d(auc));
                         }
                     }
-                    // sums of terms >= 0: their bits tell zero from more without the f64 pipe
-                    if (i > 0 && v != src && __double_as_longlong(below) > 0ll)
+                    // by their bits, without the f64 pipe
+                    if (i > 0 && v != src && positive(below))
                         atomicAdd(out + ((size_t)3 * K + k) * N + v, below);
                     if (pp >= 0 && __double_as_longlong(total) != 0ll) atomicAdd(&acc[(size_t)pp * K + k], total);
                 }

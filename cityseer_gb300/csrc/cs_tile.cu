@@ -1073,9 +1073,11 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
                         row[0] = dep;
                         row[32] = depb;
                     }
-                    // a source credits a node only with what is positive, as the reference does per source
-                    if (src || !on || !positive(acc)) acc = 0.0;
-                    if (src || !on || !positive(accb)) accb = 0.0;
+                    // a source credits a node only with what is positive, as the reference does per source (its
+                    // dependency - seed is NaN at a destination whose trips have no finite weight)
+                    const bool credited = on && !src && (!OD || fabsf(pairf) < inf_f());
+                    if (!credited || !positive(acc)) acc = 0.0;
+                    if (!credited || !positive(accb)) accb = 0.0;
                     if (!unit) {
                         if (!is_zero(acc)) acc = __dmul_rn(acc, f2d(wt));
                         if (!is_zero(accb)) accb = __dmul_rn(accb, f2d(wt));

@@ -1,4 +1,4 @@
-"""Trip weights of either sign, in each schedule of the shortest-path kernels: one warp per source, one
+"""Trip weights of any value, in each schedule of the shortest-path kernels: one warp per source, one
 block per source, and tiles of 32 sources (which calls of 10,000 sources of this reach take by themselves)."""
 import numpy as np
 import pytest
@@ -66,3 +66,26 @@ def test_trips_of_both_signs(lattice, schedule, monkeypatch):
     for m, name in enumerate(("node_betweenness", "node_betweenness_beta")):
         for i, dist in enumerate(d):
             assert_close_sums(getattr(res, name)[dist], ref[m, i], rtol=1e-9, atol=1e-9, what=f"{schedule} {name}[{dist}]")
+
+
+@pytest.mark.parametrize("schedule", ["warp", "tile"])
+def test_trips_without_a_finite_weight(lattice, schedule, monkeypatch):
+    """Trips of weight NaN or infinity leave NaN in no row; the block kernel's rows are the measure."""
+    n = lattice.node_bound()
+
+    def weights(rng, m):
+        w = rng.uniform(0.5, 5.0, m)
+        w[rng.choice(m, 30, replace=False)] = np.nan
+        w[rng.choice(m, 30, replace=False)] = np.inf
+        return w
+
+    od = _trips(n, weights)
+    _choose(monkeypatch, "block")
+    want = lattice.betweenness_od_shortest(od, distances=DISTANCES)
+    _choose(monkeypatch, schedule)
+    got = lattice.betweenness_od_shortest(od, distances=DISTANCES)
+    for name in ("node_betweenness", "node_betweenness_beta"):
+        for dist in DISTANCES:
+            a, b = getattr(got, name)[dist], getattr(want, name)[dist]
+            assert not np.isnan(a).any() and np.isfinite(b).sum() > n // 2
+            assert_close_sums(a, b, rtol=1e-9, atol=1e-9, what=f"{schedule} {name}[{dist}]")
