@@ -393,10 +393,13 @@ __device__ void adjacency(const Params &p, const Arrays &a, const Smem &sm, cons
             a.node[i] = n;
         }
     }
-    if (bad) v.fail = 1;
     if (unpaired) p.hdr->pad[UNPAIRED_SLOT] = 1ull;
-    __syncthreads();
-    if (v.fail) return;
+    // every thread takes the same way on: a flag read after the barrier could be one set beyond it
+    if (__syncthreads_or(bad)) {
+        if (threadIdx.x == 0) v.fail = 1;
+        __syncthreads();
+        return;
+    }
     for (int i0 = (threadIdx.x >> 5) * 4; i0 < R; i0 += NW * 4) {
         const int i = i0 + (lane >> 3);
         Node n{0u, 0u, 0, 0u};
