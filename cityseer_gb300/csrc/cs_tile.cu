@@ -1221,6 +1221,7 @@ __device__ __forceinline__ void flush_counts(WsHeader *h, const Vars &v, const C
     atomicAdd(&h->edges_relaxed, v.relaxed);
     atomicAdd(&h->nodes_settled, v.settled);
     atomicAdd(&h->sources_done, n.done);
+    atomicAdd(&h->pad[SERVED_SLOT], n.done);
     for (int q = 0; q < 7; q++) atomicAdd(&h->pad[q], (unsigned long long)n.ph[q]);
 }
 

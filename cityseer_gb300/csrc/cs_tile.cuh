@@ -15,6 +15,7 @@ constexpr int NW = TPB / 32;    // warps per block
 constexpr int BPSM = 2;         // resident blocks per SM
 constexpr int PMAX = 8;         // out-edges per node (the graph's maximum out-degree)
 constexpr int MMAX = 65536;     // nodes of one tile (dirty bits live in shared memory)
+constexpr int SERVED_SLOT = 11; // header word: sources whose rows the tile kernel wrote itself
 
 // Per-block scratch: offsets of its arrays, each indexed by the tile's node number.
 struct Geometry {

@@ -349,10 +349,14 @@ cs_status cs_batch_failed(void *workspace_dev, const cs_plan *plan, int32_t *ite
 cs_status cs_last_counters(int64_t *sources, int64_t *edges_relaxed, int64_t *nodes_settled, int64_t *launches);
 
 /* Per-phase SM cycles of the last call on this thread, summed over warps: 0 search, 1 sort,
- * 2 predecessor replay, 3 closeness, 4 sigma, 5 backward sweep, 6 scratch reset.  After a
+ * 2 predecessor replay, 3 closeness, 4 sigma, 5 backward sweep, 6 scratch reset.  In tiles of 32
+ * sources, summed over blocks: 0 union search, 1 adjacency, 2 search, 3 replay, 4 schedule and path
+ * counts, 5 closeness, 6 backward sweep.  After a
  * simplest-path call: 0 search, 1 sort, 2 replay, 3 node best + closeness, 4 backward sweep,
  * 5 scratch reset, 6 exact heap search; 7 holds the number of replay rounds instead.  Entries 8-15
- * (n <= 16) are diagnostics: 8 the live progress count; after a simplest-path call 9-11 the
+ * (n <= 16) are diagnostics: 8 the live progress count; after a shortest-path call or batch 11 the
+ * sources that tiles served (the others ran one block or warp each) and, after a batch, 10 those that
+ * its last tiled launch left to the per-warp kernel; after a simplest-path call 9-11 the
  * replayed states whose route came out below / above their search key / unreached, 12-14 the
  * replay rounds that ended with the routes out of order / an unreached state offered to / a state
  * reached outside the search's set, 15 the states that later replay rounds kept from the round

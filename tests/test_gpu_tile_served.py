@@ -4,8 +4,10 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from cityseer_gb300 import _native, synth
+import oracle
+from cityseer_gb300 import _native, abi, centrality, common, device, synth
 from cityseer_gb300.graph import NetworkStructure
+from helpers import assert_close_sums
 
 pytestmark = pytest.mark.gpu
 
@@ -24,6 +26,13 @@ def _left() -> int:
     left = C.c_int64()
     _native.check(_native.load().cs_last_retries(C.byref(left), None), "cs_last_retries")
     return left.value
+
+
+def _served() -> int:
+    """Sources of the last call whose rows came from tiles."""
+    entries = (C.c_int64 * 16)()
+    _native.check(_native.load().cs_last_phase_cycles(entries, 16), "cs_last_phase_cycles")
+    return entries[11]
 
 
 def _per_warp(ns, monkeypatch, distances):
@@ -56,3 +65,74 @@ def test_one_way_loops(monkeypatch):
     got = ns.centrality_shortest(distances=DISTANCES)
     assert _left() > 0
     _same(got, _per_warp(ns, monkeypatch, DISTANCES))
+
+
+@pytest.fixture(scope="module")
+def lattice():
+    return synth.primal_structure(_streets())
+
+
+@pytest.mark.parametrize("distances,kw", [
+    ([700, 2400, 4000], {}),  # unions of up to 5,000 nodes
+    ([2400], dict(tolerance=2.0)),
+    ([2400], dict(compute_closeness=False)),
+])
+def test_every_source_against_the_oracle(lattice, distances, kw):
+    """Counts are exact, betweenness differs in the order of its f64 sums, closeness also in the last bits
+    of its f32 exponentials and quotients."""
+    n = lattice.node_bound()
+    d, b, s = common.pair_distances_betas_time(1.33333, distances=distances)
+    closeness = kw.get("compute_closeness", True)
+    ref, _ = oracle.centrality_shortest(oracle.OracleGraph(lattice), d, b, s, closeness=closeness,
+                                        tol=centrality.validate_tolerance(kw.get("tolerance")),
+                                        plan=oracle.plan_from(centrality.prepare_source_sampling(
+                                            lattice, None, None, None, None), n),
+                                        nthreads=oracle.default_threads())
+    res = lattice.centrality_shortest(distances=distances, **kw)
+    assert (_served(), _left()) == (n, 0)
+    for m, name in enumerate(ROWS):
+        if m < 5 and not closeness:
+            continue
+        for i, dist in enumerate(d):
+            got = getattr(res, name)[dist]
+            if name in ("node_density", "node_cycles"):
+                np.testing.assert_array_equal(got, ref[m, i], err_msg=f"{name}[{dist}]")
+            else:
+                assert_close_sums(got, ref[m, i], rtol=1e-9 if m >= 5 else 1e-5, what=f"{name}[{dist}]")
+
+
+def test_trips_of_every_node_against_the_oracle(lattice):
+    n = lattice.node_bound()
+    rng = np.random.default_rng(9)
+    o = np.repeat(np.arange(n), 2)
+    od = centrality.OdMatrix(o, np.clip(o + rng.integers(-900, 900, len(o)), 0, n - 1), rng.uniform(0.1, 9.0, len(o)))
+    d, b, s = common.pair_distances_betas_time(1.33333, distances=DISTANCES)
+    ref = oracle.betweenness_od(oracle.OracleGraph(lattice), d, b, s, od.rows(n), ns=lattice,
+                                nthreads=oracle.default_threads())
+    res = lattice.betweenness_od_shortest(od, distances=DISTANCES)
+    assert (_served(), _left()) == (n, 0)
+    for m, name in enumerate(("node_betweenness", "node_betweenness_beta")):
+        for i, dist in enumerate(d):
+            assert_close_sums(getattr(res, name)[dist], ref[m, i], rtol=1e-9, what=f"{name}[{dist}]")
+
+
+def test_unions_beyond_the_scratch(lattice, monkeypatch):
+    """A plan of small capacity: the tiles' unions outgrow it, their sources go to the per-warp kernel and
+    its capacity chain, and the scratch is clean for the next call, whose tiles fit."""
+    n = lattice.node_bound()
+    for distances, left in (([2400], n), ([400], 0)):
+        call = abi.shortest_call(lattice, distances)
+        if left:
+            plan = device.plan_primal(centrality._primal_csr(lattice), 0, 1, 1.33333, cap=256, mem_budget=8 << 30)
+            ws = device.Workspace(plan, n, call.out.device)
+        else:
+            monkeypatch.setenv("CS_TILE", "1")  # few hops: not by the rule
+        call.plan, call.workspace = plan, ws
+        abi.check(abi.library().cs_centrality_shortest(*call.args()))
+        served = _served()
+        got = call.out.cpu().numpy()
+        assert served == n - left and (_left() > 0) == (left > 0)
+        want = _per_warp(lattice, monkeypatch, distances)
+        for m, name in enumerate(ROWS):
+            col = getattr(want, name)[distances[0]]
+            assert np.linalg.norm(got[m, 0] - col) <= 1e-10 * np.linalg.norm(col), (name, distances)
