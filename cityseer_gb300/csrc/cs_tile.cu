@@ -102,7 +102,12 @@ struct Smem {
     uint32_t *bits, *part;
 };
 
-size_t smem_bytes(int k, int mcap) { return ((sizeof(Vars) + 15) & ~size_t(15)) + 3 * 128 * (size_t)k + 2 * ((size_t)mcap / 8); }
+constexpr size_t smem_bytes(int k, int mcap) {
+    return ((sizeof(Vars) + 15) & ~size_t(15)) + 3 * 128 * (size_t)k + 2 * ((size_t)mcap / 8);
+}
+// No launch asks for more than a kernel may have without an attribute, which would be the kernel's and
+// not the launch's: another thread could change it between a call's setting and its launch.
+static_assert(smem_bytes(MAXK, MMAX) + sizeof(Params) <= 48 * 1024, "a launch needs more shared memory than the default");
 
 __device__ __forceinline__ Smem smem(char *raw, int k, int mcap) {
     char *c = raw + ((sizeof(Vars) + 15) & ~size_t(15));
@@ -1370,10 +1375,7 @@ Geometry geometry(size_t region_bytes, int k, const float *dk, bool od) {
 
 template <bool OD>
 cudaError_t launch_t(const Params &p, int blocks, cudaStream_t stream) {
-    const size_t bytes = smem_bytes(p.k, p.geo.mcap);
-    const cudaError_t e = cudaFuncSetAttribute(tile_kernel<OD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    tile_kernel<OD><<<blocks, TPB, bytes, stream>>>(p);
+    tile_kernel<OD><<<blocks, TPB, smem_bytes(p.k, p.geo.mcap), stream>>>(p);
     return cudaGetLastError();
 }
 
@@ -1383,10 +1385,7 @@ cudaError_t launch(const Params &p, bool od, int blocks, cudaStream_t stream) {
 
 cudaError_t launch_batch(const Params &p, const cs_batch_job *jobs_dev, int lo, int hi, int kmax, int blocks,
                          cudaStream_t stream) {
-    const size_t bytes = smem_bytes(kmax, p.geo.mcap);
-    const cudaError_t e = cudaFuncSetAttribute(tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    tile_batch_kernel<<<blocks, TPB, bytes, stream>>>(p, jobs_dev, lo, hi, kmax);
+    tile_batch_kernel<<<blocks, TPB, smem_bytes(kmax, p.geo.mcap), stream>>>(p, jobs_dev, lo, hi, kmax);
     return cudaGetLastError();
 }
 
