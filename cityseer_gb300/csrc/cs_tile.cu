@@ -222,20 +222,22 @@ __device__ int collect(uint32_t *bits, int n_bits, int *list, int cmax, int *wsu
 // Sums over a warp without f64 adds.  GB300 runs f64 at 1/64 of the f32 rate: the five shuffled f64 adds
 // of a warp sum hold an SM's f64 pipe for 80 cycles.  Instead the terms (nonnegative, finite) become fixed
 // point at the largest term's exponent, integer warp reductions add them, and the total goes back to f64
-// by integer arithmetic.  A sum of f32 terms keeps 48 bits below the largest term's top bit, so it is
-// exact while the terms span at most 24 binary orders; a sum of f64 terms keeps 59.
-__device__ __forceinline__ FixSum fix_sum(float x) {  // bias 174
+// by integer arithmetic.  A sum of f32 terms keeps 54 bits from the largest term's top bit down, so it is
+// exact while the terms span at most 30 binary orders, and beyond loses less than f64 adds of them (1,500
+// sums of terms over 60 orders: 4.3e-16 at most, f64 5.4e-16); a sum of f64 terms keeps 59.
+constexpr int BIAS_F = 180, BIAS_D = 1081;
+__device__ __forceinline__ FixSum fix_sum(float x) {  // BIAS_F
     const uint32_t b = __float_as_uint(x);
     const uint32_t top = __reduce_max_sync(FULL, b);
     if (top >= 0x7f800000u) return {0ull, -1};
     const int e = max((int)(b >> 23), 1), emax = max((int)(top >> 23), 1);
     const uint32_t m = (b & 0x7fffffu) | (b >= 0x800000u ? 0x800000u : 0u);
-    const unsigned long long t = ((unsigned long long)m << 24) >> min(emax - e, 63);
-    const unsigned lo = __reduce_add_sync(FULL, (unsigned)t & 0xffffffu);
-    const unsigned hi = __reduce_add_sync(FULL, (unsigned)(t >> 24));
-    return {((unsigned long long)hi << 24) + lo, emax};
+    const unsigned long long t = ((((unsigned long long)m << 31) >> min(emax - e, 63)) + 1ull) >> 1;  // to nearest
+    const unsigned lo = __reduce_add_sync(FULL, (unsigned)t & 0x7ffffffu);
+    const unsigned hi = __reduce_add_sync(FULL, (unsigned)(t >> 27));
+    return {((unsigned long long)hi << 27) + lo, emax};
 }
-__device__ __forceinline__ FixSum fix_sum(double x) {  // bias 1081
+__device__ __forceinline__ FixSum fix_sum(double x) {  // BIAS_D
     const uint32_t h = (uint32_t)__double2hiint(x);
     const uint32_t top = __reduce_max_sync(FULL, h);
     if (top >= 0x7ff00000u) return {0ull, -1};
@@ -957,14 +959,14 @@ __device__ void closeness(const Params &p, const Arrays &a, const Smem &sm) {
             keep(1, in ? fmul(expf(fmul(-p.beta[k], c)), wt) : 0.0f);
             if (fresh) {
                 if (unit) {
-                    if (lane == 2) mys = FixSum{(unsigned long long)__popc(fresh), 174};
+                    if (lane == 2) mys = FixSum{(unsigned long long)__popc(fresh), BIAS_F};
                 } else {
                     keep(2, mine ? wt : 0.0f);
                 }
                 keep(3, mine ? far : 0.0f);
                 keep(4, mine ? har : 0.0f);
             }
-            const double val = mys.e < 0 ? slow : fix_to_d(mys, 174);
+            const double val = mys.e < 0 ? slow : fix_to_d(mys, BIAS_F);
             if (__double_as_longlong(val) == 0ll) continue;
             double *dst = (lane < 2) ? p.out + (lane == 0 ? 2 : 4) * KN : p.bucket + (size_t)(lane - 2) * KN;
             atomicAdd(dst + (size_t)k * N + t, val);
@@ -1091,7 +1093,7 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
                         if (!is_zero(accb)) accb = __dmul_rn(accb, f2d(wt));
                     }
                     const FixSum s0 = fix_sum(acc), s1 = fix_sum(accb);
-                    double val = fix_to_d(lane ? s1 : s0, 1081);
+                    double val = fix_to_d(lane ? s1 : s0, BIAS_D);
                     if ((s0.e < 64 && (s0.e < 0 || s0.sum)) || (s1.e < 64 && (s1.e < 0 || s1.sum))) {
                         // not finite, of a negative source weight, or close to the smallest f64
                         const double d0 = slow_sum(acc), d1 = slow_sum(accb);

@@ -1,12 +1,20 @@
-"""Trip weights of any value, in each schedule of the shortest-path kernels: one warp per source, one
-block per source, and tiles of 32 sources (which calls of 10,000 sources of this reach take by themselves)."""
+"""Source and trip weights of any sign and size, in each schedule of the shortest-path kernels: one warp
+per source, one block per source, and tiles of 32 sources (which calls of 10,000 sources of this reach
+take by themselves)."""
+import ctypes as C
+import math
+
 import numpy as np
 import pytest
 import torch
+from scipy.sparse import coo_matrix
+from scipy.sparse.csgraph import connected_components
 
 import oracle
 from cityseer_gb300 import _native, common, synth
+from cityseer_gb300.batch import Batch
 from cityseer_gb300.centrality import OdMatrix
+from cityseer_gb300.graph import NetworkStructure
 from helpers import assert_close_sums
 
 pytestmark = pytest.mark.gpu
@@ -89,3 +97,26 @@ def test_trips_without_a_finite_weight(lattice, schedule, monkeypatch):
             a, b = getattr(got, name)[dist], getattr(want, name)[dist]
             assert not np.isnan(a).any() and np.isfinite(b).sum() > n // 2
             assert_close_sums(a, b, rtol=1e-9, atol=1e-9, what=f"{schedule} {name}[{dist}]")
+
+
+def test_tile_sums_keep_every_bit_of_small_terms(monkeypatch):
+    """One source of weight 1 among sources of about 1e-9: a tile's sums of 32 terms are as exact as f64
+    adds of them, and the tiles' sums (and the sources that tiles leave) are added in f64: at most
+    32 + 32 + left roundings of 2^-53."""
+    p = synth.lattice(side=32, spacing=80.0, jitter=15.0, drop=0.1, seed=5)
+    n = 32 * 32
+    w = np.random.default_rng(8).uniform(0.5e-9, 1.5e-9, n).astype(np.float32)
+    w[527] = 1.0
+    src, dst = np.concatenate([p.u, p.v]), np.concatenate([p.v, p.u])
+    ns = NetworkStructure.from_arrays(p.x, p.y, src, dst, np.concatenate([p.length, p.length]), weight=w)
+    monkeypatch.setenv("CS_TILE", "1")
+    batch = Batch([dict(ns=ns, mode="shortest", distances=[6000])])  # to every node of the component
+    batch.run()
+    entries = (C.c_int64 * 16)()
+    _native.check(_native.load().cs_last_phase_cycles(entries, 16), "cs_last_phase_cycles")
+    served = entries[11]
+    assert served > n // 2
+    got = batch.results()[0].node_density[6000]
+    _, part = connected_components(coo_matrix((np.ones(len(src)), (src, dst)), shape=(n, n)), directed=False)
+    want = np.array([math.fsum(float(w[i]) for i in np.nonzero(part == part[v])[0] if i != v) for v in range(n)])
+    assert np.all(np.abs(got - want) <= (64 + n - served) * 2.0 ** -53 * want)
