@@ -22,6 +22,8 @@ CS_ERR_TIMEOUT = 4
 CS_ERR_INTERNAL = 5
 CS_BATCH_ASYNC = 1
 CS_BATCH_NEAR_SOURCES = 2
+CS_PLAN_NEAR_SOURCES = 0x100
+CS_TILE_SOURCES_MIN = 8192
 
 _ptr = C.c_void_p
 

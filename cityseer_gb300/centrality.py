@@ -281,7 +281,7 @@ def _hilbert_rank(ns) -> np.ndarray:
     return rank
 
 
-TILE_CALL = 8192  # no smaller call has a tile of 32 sources for every resident block
+TILE_CALL = _native.CS_TILE_SOURCES_MIN  # no smaller call is served in tiles
 
 
 def spatial_order(ns, process: np.ndarray, fewest: int = TILE_CALL) -> np.ndarray:
@@ -367,6 +367,7 @@ def _workspace(ns, csr, mode: int, k: int, speed: float, max_seconds: int | None
         del ws
     torch.cuda.empty_cache()
     plan = device.plan_primal(csr, 0, (need_l + 1) // 2, speed, cap=cap, mem_budget=_mem_budget(csr.device))
+    plan.variant |= _native.CS_PLAN_NEAR_SOURCES  # the calls on it list their sources by spatial_order
     ws = device.Workspace(plan, csr.n_bound, csr.device)
     ns._cache["ws"] = ws
     return ws

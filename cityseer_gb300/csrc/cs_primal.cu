@@ -246,7 +246,8 @@ cs_status validate_primal(const cs_primal_graph *g) {
 // dependency pass outweighing the extra warps), 4 for segments, trees and accessibility (segment
 // centrality on the 250x250 curved lattice: 2.67M sources/s against 2.49M with 3).
 int requested_variant(const cs_plan *plan) {
-    if (plan && plan->variant >= 2 && plan->variant <= 4) return plan->variant;
+    const int v = plan ? plan->variant & 0xff : 0;
+    if (v >= 2 && v <= 4) return v;
     const char *e = getenv("CS_MIN_BLOCKS_PER_SM");
     return (e && e[0] >= '2' && e[0] <= '4') ? e[0] - '0' : 0;
 }
@@ -300,26 +301,35 @@ bool block_schedule(long long n_src, float maxsec, float delta) {
 // Tile kernel (cs_tile.cu): 32 nearby sources per block, one per lane.  A tile does its sources' common
 // work once, over the union of their reaches, so it pays where the reach is much wider than the tile and
 // there is a tile for every resident block:
-//  - 32 sources for each of the 2 blocks per SM (9,728 on 152 SMs);
+//  - the caller vouches for the sources' order (CS_PLAN_NEAR_SOURCES);
+//  - 32 sources for each of the 2 blocks per SM (9,728 on 152 SMs), and CS_TILE_SOURCES_MIN;
 //  - hops to the cutoff (seconds / median edge seconds, half a plan's band width) at least 5 times the
 //    tile's radius sqrt(16 N / sources) in hops.
 // Measured on lattices against one warp per source: 5 km at 80 m (62 hops), every node a source 70 ms
 // against 146 (90,000 nodes), one node in nine 17.5 against 19.6, one in eighteen 16.7 against 12.4;
 // 3.2 km at 100 m (32 hops), every node (19,600) 6.1 against 8.7, every second 4.4 against 5.0, every
 // fourth 4.1 against 3.2; 1.6 km (16 hops) 3.3 against 3.2; 500 m at 80 m 4.8 against 3.5.
+// By the sources' order, tiles against warps, every node: 202,500 nodes to 5 km along a curve 169 ms against
+// 297, in rows 255 against 301, at random 359 against 345; 19,881 nodes to 3.2 km 8.9 against 11.1, 14.7
+// against 11.0 and 13.9 against 13.2.
+// Trips (all origins, 3 to 9 trips each): 10,000 origins to 3.2 km 4.6 ms against 5.4, 40,000 to 5 km 27.4
+// against 45.6, to 3.2 km 17.0 against 22.8; 22,500 and 10,000 origins of 90,000 and 40,000 nodes, beyond
+// the rule, 16.5 against 14.7 and 8.3 against 7.1.
 // CS_TILE=0 leaves every source to the other kernels, CS_TILE=1 takes every call the kernel can serve.
-long long tile_call() { return 32ll * cs::tile::BPSM * std::max(1, sm_count()); }
+long long tile_call() {
+    return std::max<long long>(CS_TILE_SOURCES_MIN, 32ll * cs::tile::BPSM * std::max(1, sm_count()));
+}
 bool tile_reach(long long n_src, int n_bound, float maxsec, float delta) {
     if (!(delta > 0.0f)) return false;
     const double hops = 2.0 * maxsec / delta, radius = std::sqrt(16.0 * n_bound / (double)n_src);
     return hops >= 5.0 * radius;
 }
 // Returns the sources per tile, 0: not this kernel.
-int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float delta) {
+int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float delta, bool near) {
     const char *e = getenv("CS_TILE");
     if (e && e[0] == '0') return 0;
     if (e && e[0] == '1') return (int)std::max(1ll, std::min(32ll, (n_src + blocks - 1) / blocks));
-    return n_src >= tile_call() && tile_reach(n_src, n_bound, maxsec, delta) ? 32 : 0;
+    return near && n_src >= tile_call() && tile_reach(n_src, n_bound, maxsec, delta) ? 32 : 0;
 }
 
 // The shortest-path jobs of a batch that go to the tile kernel: the rule's reach for each job by itself, its
@@ -588,7 +598,8 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
     int tile_blocks = 0, lanes = 0;
     if ((mode == cs::MODE_SHORTEST || mode == cs::MODE_OD) && P <= cs::tile::PMAX) {
         tile_blocks = std::max(1, std::min(sm_count() * cs::tile::BPSM, plan->n_slots));
-        lanes = tile_lanes(p.n_src, tile_blocks, g->n_bound, p.maxsec, plan->delta_seconds);
+        lanes = tile_lanes(p.n_src, tile_blocks, g->n_bound, p.maxsec, plan->delta_seconds,
+                           (plan->variant & CS_PLAN_NEAR_SOURCES) != 0);
         if (lanes > 0) {
             tile_blocks = (int)std::min<long long>(tile_blocks, (p.n_src + lanes - 1) / lanes);
             geo = cs::tile::geometry((lay.compact_total / tile_blocks) & ~size_t(255), K, p.dk, mode == cs::MODE_OD);

@@ -135,13 +135,22 @@ typedef struct {
     int32_t lanes;        /* accumulator lanes per reached node */
     int32_t variant;      /* register budget: 2, 3 or 4 resident 256-thread blocks per SM for every
                            * launch; 0 (default): slots sized for 4, and each launch takes 3 for
-                           * shortest-path and OD centrality, 4 for segments, trees and accessibility */
+                           * shortest-path and OD centrality, 4 for segments, trees and accessibility;
+                           * the caller may add CS_PLAN_NEAR_SOURCES after planning */
     int32_t max_degree;   /* batches: largest out-degree over the jobs */
     int32_t n_bound;      /* node bound the slot geometry was sized for (set by the planners) */
     int32_t cta_blocks;   /* shortest-path plans: blocks of the block-per-source kernel whose scratch
                              the workspace holds (0: the per-warp kernel serves every source) */
     size_t workspace_bytes;
 } cs_plan;
+
+/* Added to a plan's variant: in this plan's shortest-path and OD calls of CS_TILE_SOURCES_MIN sources or
+ * more, consecutive entries of sources_dev lie near one another (on a space-filling curve, say).  Calls of
+ * wide reach then search for 32 of them at once.  Sources in another order (rows of a grid, or at random)
+ * are faster one by one, as calls without the flag run them. */
+#define CS_PLAN_NEAR_SOURCES 0x100
+/* No smaller call is served in tiles of 32 sources (unless CS_TILE=1 asks for them). */
+#define CS_TILE_SOURCES_MIN 8192
 
 /* One job of a batched launch: a graph, a mode (0 shortest, 1 segment, 3 both from one search per
  * source), its thresholds, sources and outputs.  Many jobs of
