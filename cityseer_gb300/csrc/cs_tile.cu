@@ -64,7 +64,10 @@ constexpr int LIST = 256;         // candidates of one schedule step
 // The union search only orders and bounds the tile: wider bands than a search's (fewer rounds, each a
 // chain of loads and barriers) suit it; 2x and 4x took 2.2 and 3.0 of a city pass's 175 ms off.
 constexpr float UNION_BAND = 4.0f;
-constexpr int UNPAIRED_SLOT = 9;  // header word: the graph has an edge without one back
+// Header words: one bit per job of a batch (a plain call is job 0; the 513th job shares the first one's),
+// set when its graph turns out to have an edge without one back.  No tile of it can be served.
+constexpr int UNPAIRED_SLOT = 16, UNPAIRED_WORDS = 8;
+static_assert(UNPAIRED_SLOT + UNPAIRED_WORDS <= 24, "beyond the header");
 constexpr int PART = 16;          // partly ready nodes that each step lets go
 constexpr int MAX_ROUNDS = 1 << 17;  // bounded loops (never reached on a consistent graph)
 constexpr float TIE_WINDOW = 1.00115f;  // offers above best * this cannot stay predecessors (8 steps of 1e-4)
@@ -85,6 +88,7 @@ struct Vars {
     long long base;
     unsigned herr;
     int nl;
+    int job;
     unsigned long long settled, relaxed;
     int wsum[NW + 1];
     int src[32], loc[32];
@@ -371,6 +375,14 @@ __device__ void discover(const Params &p, const Arrays &a, const Smem &sm, float
     __syncthreads();
 }
 
+__device__ __forceinline__ unsigned long long *unpaired_word(WsHeader *h, int job) {
+    return &h->pad[UNPAIRED_SLOT + (job >> 6) % UNPAIRED_WORDS];
+}
+__device__ __forceinline__ void mark_unpaired(WsHeader *h, int job) { atomicOr(unpaired_word(h, job), 1ull << (job & 63)); }
+__device__ __forceinline__ int is_unpaired(WsHeader *h, int job) {
+    return (int)((__ldcg(unpaired_word(h, job)) >> (job & 63)) & 1ull);
+}
+
 // Eight lanes per node, one per edge.
 __device__ void adjacency(const Params &p, const Arrays &a, const Smem &sm, const float *d1, const uint32_t *aux) {
     Vars &v = sm.v;
@@ -400,7 +412,7 @@ __device__ void adjacency(const Params &p, const Arrays &a, const Smem &sm, cons
             a.node[i] = n;
         }
     }
-    if (unpaired) p.hdr->pad[UNPAIRED_SLOT] = 1ull;
+    if (unpaired) mark_unpaired(p.hdr, v.job);
     // every thread takes the same way on: a flag read after the barrier could be one set beyond it
     if (__syncthreads_or(bad)) {
         if (threadIdx.x == 0) v.fail = 1;
@@ -448,7 +460,7 @@ __device__ void adjacency(const Params &p, const Arrays &a, const Smem &sm, cons
         if (i < R) a.adj[(size_t)i * PMAX + j] = e;
     }
     if (bad) v.fail = 1;
-    if (unpaired) p.hdr->pad[UNPAIRED_SLOT] = 1ull;
+    if (unpaired) mark_unpaired(p.hdr, v.job);
     __syncthreads();
 }
 
@@ -1241,12 +1253,15 @@ __global__ void __launch_bounds__(TPB, BPSM) tile_kernel(const __grid_constant__
     float *d1 = (float *)(p.dense + p.dense_stride * (size_t)blockIdx.x);
     uint32_t *aux = (uint32_t *)(p.dense + p.dense_stride * (size_t)blockIdx.x + p.aux_off);
     Counts n;
-    if (threadIdx.x == 0) v.settled = v.relaxed = 0ull;
+    if (threadIdx.x == 0) {
+        v.settled = v.relaxed = 0ull;
+        v.job = 0;
+    }
     while (true) {
         if (threadIdx.x == 0) {
             v.base = (long long)atomicAdd(&p.hdr->work_next, 1ull) * p.lanes;
             v.herr = __ldcg(&p.hdr->err);
-            v.fail = __ldcg(&p.hdr->pad[UNPAIRED_SLOT]) != 0ull;  // then no tile can be served here
+            v.fail = is_unpaired(p.hdr, 0);
         }
         __syncthreads();
         const long long base = v.base;
@@ -1278,7 +1293,6 @@ __global__ void __launch_bounds__(TPB, BPSM) tile_batch_kernel(const __grid_cons
         if (threadIdx.x == 0) {
             const long long t = (long long)atomicAdd(&base.hdr->work_next, 1ull);
             v.herr = __ldcg(&base.hdr->err);
-            v.fail = __ldcg(&base.hdr->pad[UNPAIRED_SLOT]) != 0ull;
             int j = cur;
             while (j < hi && t >= before) {
                 j++;
@@ -1323,6 +1337,8 @@ __global__ void __launch_bounds__(TPB, BPSM) tile_batch_kernel(const __grid_cons
                     cur = j;
                 }
                 v.base = (t - first) * 32;
+                v.job = j;
+                v.fail = is_unpaired(base.hdr, j);
             }
         }
         __syncthreads();

@@ -7,6 +7,7 @@ import torch
 
 import oracle
 from cityseer_gb300 import _native, abi, centrality, common, device, synth
+from cityseer_gb300.batch import Batch
 from cityseer_gb300.graph import NetworkStructure
 from helpers import assert_close_sums
 
@@ -18,8 +19,8 @@ SIDE = 100
 DISTANCES = [700, 2400]
 
 
-def _streets():
-    return synth.lattice(side=SIDE, spacing=80.0, jitter=15.0, drop=0.1, seed=11)
+def _streets(side=SIDE):
+    return synth.lattice(side=side, spacing=80.0, jitter=15.0, drop=0.1, seed=11)
 
 
 def _left() -> int:
@@ -51,18 +52,23 @@ def _same(got, want, names=ROWS):
             assert np.linalg.norm(getattr(got, name)[d] - col) <= 1e-10 * np.linalg.norm(col), (name, d)
 
 
-def test_one_way_loops(monkeypatch):
-    """Nodes with as many edges in as out, but no edge back for some: the tiles that meet one find out in
-    their second pass over the edges, and leave every source to the per-warp kernel."""
-    p = _streets()
-    at = SIDE * np.arange(20, 80, 12)[:, None] + np.arange(20, 80, 12)
+def _with_loops(side=SIDE):
+    """One-way loops of three streets: nodes with as many edges in as out, but no edge back for some."""
+    p = _streets(side)
+    at = side * np.arange(side // 5, side - side // 5, 12)[:, None] + np.arange(side // 5, side - side // 5, 12)
     a = at.reshape(-1)
-    b, c = a + 2, a + 2 * SIDE + 1
+    b, c = a + 2, a + 2 * side + 1
     src = np.concatenate([p.u, p.v, a, b, c])
     dst = np.concatenate([p.v, p.u, b, c, a])
     ln = np.concatenate([p.length, p.length, np.full(3 * len(a), 170.0)]).astype(np.float32)
     idx = np.concatenate([np.zeros(2 * len(p.u), np.int64), 1 + np.arange(3 * len(a))])
-    ns = NetworkStructure.from_arrays(p.x, p.y, src, dst, ln, edge_idx=idx)
+    return NetworkStructure.from_arrays(p.x, p.y, src, dst, ln, edge_idx=idx)
+
+
+def test_one_way_loops(monkeypatch):
+    """The tiles that meet an edge without one back find out in their second pass over the edges, and leave
+    every source to the per-warp kernel."""
+    ns = _with_loops()
     got = ns.centrality_shortest(distances=DISTANCES)
     assert _left() > 0
     _same(got, _per_warp(ns, monkeypatch, DISTANCES))
@@ -154,3 +160,19 @@ def test_only_vouched_orders_are_tiled(lattice, order):
     call.plan = plan
     abi.check(abi.library().cs_centrality_shortest(*call.args()))
     assert _served() == (n if order == "curve" else 0)
+
+
+def test_one_way_loops_of_one_job_of_a_batch(lattice, monkeypatch):
+    """The other jobs' sources stay in tiles (the job with the loops comes first: it reaches farthest)."""
+    loops = _with_loops(40)
+    jobs = [dict(ns=g, mode="shortest", distances=[d]) for g, d in ((loops, 1500), (lattice, 2400), (loops, 3000))]
+    batch = Batch(jobs)
+    batch.run()
+    entries = (C.c_int64 * 16)()
+    _native.check(_native.load().cs_last_phase_cycles(entries, 16), "cs_last_phase_cycles")
+    assert entries[11] >= lattice.node_bound() and entries[10] > 0
+    monkeypatch.setenv("CS_TILE", "0")
+    plain = Batch(jobs)
+    plain.run()
+    for got, want in zip(batch.results(), plain.results()):
+        _same(got, want)
