@@ -182,8 +182,11 @@ def prepare_source_sampling(ns, sample_probability, sampling_weights, random_see
         raise ValueError("source_indices and sampling_weights are mutually exclusive")
     exists = a["node_exists"]
     if source_indices is not None:
-        src = np.asarray(source_indices if isinstance(source_indices, np.ndarray) else list(source_indices),
-                         dtype=np.int64).reshape(-1)
+        plain = type(source_indices) is np.ndarray and source_indices.ndim == 1 and source_indices.dtype.kind == "i"
+        src = np.asarray(source_indices if plain else list(source_indices), dtype=np.int64)
+        if src.size != len(src):
+            raise ValueError("source_indices must hold one node index per entry")
+        src = src.reshape(-1)
         bad = (src < 0) | (src >= nb)
         bad[~bad] = ~exists[src[~bad]].astype(bool)
         if bad.any():
