@@ -167,7 +167,7 @@ TILE_PHASES = ("union", "adjacency", "search", "replay", "schedule", "closeness"
 WARP_PHASES = ("search", "sort", "replay", "closeness", "sigma", "backward", "reset")
 
 
-def traffic_ratio(kernel: str = "tile_kernel"):
+def traffic_ratio(kernel: str):
     """DRAM bytes per algorithmic byte of the timed kernel, from the ncu figures kept in
     profiles/traffic.json (one capture of that kernel on a smaller lattice of the same recipe)."""
     try:
@@ -297,9 +297,10 @@ def run_gpu(args):
         c = centrality.last_counters()
         counters.append(c)
         launches += c[3]
-    ph = (C.c_int64 * 8)()
-    lib.cs_last_phase_cycles(ph, 8)
-    ph = [int(x) for x in ph][:7]
+    entries = (C.c_int64 * 16)()
+    lib.cs_last_phase_cycles(entries, 16)
+    ph = [int(x) for x in entries][:7]
+    tiled = entries[11] > 0  # sources served by the tile kernel
     torch.cuda.synchronize()
     if ws > 1:
         torch.distributed.barrier()
@@ -320,13 +321,14 @@ def run_gpu(args):
     alg_bytes = 12.0 * e_relax + 24.0 * n_settled + 8.0 * 7.0 * reach_sum
     peak, peak_kind = measured_peak_hbm()
     achieved = alg_bytes / step_s / 1e9
+    ratio = traffic_ratio("tile_kernel" if tiled else "primal_sync_kernel")
     roofline = {
         "bound": "hbm",
         "achieved": achieved,
         "peak": peak,
         "unit": "GB/s",
         "frac": achieved / peak,
-        "traffic": (traffic_ratio() * alg_bytes) if traffic_ratio() else None,
+        "traffic": ratio * alg_bytes if ratio else None,
         "traffic_note": "DRAM bytes per launch: the ncu traffic per algorithmic byte of a smaller lattice "
                         "(profiles/traffic.json) times this launch's algorithmic bytes",
         "peak_kind": peak_kind,
@@ -374,7 +376,7 @@ def run_gpu(args):
             # search slots of the shortest-path launches (plans sized for the 4-block budget hold
             # more; the block-synchronous shortest-path kernel runs with 3 blocks per SM)
             "slots": int(min(wsp.plan.n_slots, lib.cs_device_sm_count() * 3 * 8)
-                         if wsp.plan.variant & 0xff == 0 else wsp.plan.n_slots),
+                         if (wsp.plan.variant & 0xff) == 0 else wsp.plan.n_slots),
             "cap": int(wsp.plan.cap),
             "delta_s": float(wsp.plan.delta_seconds),
         },
@@ -382,7 +384,7 @@ def run_gpu(args):
         "roofline": roofline,
         "gpu_launches": int(launches),
         "phase_share": {nm: round(v / max(1, sum(ph)), 4) for nm, v in
-                        zip(TILE_PHASES if n_src >= centrality.TILE_CALL else WARP_PHASES, ph)},
+                        zip(TILE_PHASES if tiled else WARP_PHASES, ph)},
         "clocks": clk,
     }
     if rank == 0 and ws == 1 and not args.no_cpu:  # the CPU baseline is reported at N = 1 only
@@ -520,6 +522,8 @@ def run_batch(args):
         r = centrality.estimate_reach(ns, csr, 1.33333, max(s))
         cap = int(min(csr.n_bound, max(1024, -(-int(r * 1.3) // 256) * 256)))
         plan = device.plan_primal(csr, mode, len(d), 1.33333, cap=cap, mem_budget=centrality._mem_budget(dev))
+        if b.flags & _native.CS_BATCH_NEAR_SOURCES:
+            plan.variant |= _native.CS_PLAN_NEAR_SOURCES  # the batch's order, vouched for in both forms
         ws_bytes = max(ws_bytes, int(plan.workspace_bytes))
         q = centrality._make_query(d, bb, s, 1.33333, float(centrality.TIE_EPSILON), True, True, False,
                                    jb["keep"][0], jb["keep"][1], jb["keep"][2])
