@@ -230,13 +230,18 @@ __device__ int collect(uint32_t *bits, int n_bits, int *list, int cmax, int *wsu
 // exact while the terms span at most 30 binary orders, and beyond loses less than f64 adds of them (1,500
 // sums of terms over 60 orders: 4.3e-16 at most, f64 5.4e-16); a sum of f64 terms keeps 59.
 constexpr int BIAS_F = 180, BIAS_D = 1081;
+__device__ __forceinline__ unsigned long long shift_right(unsigned long long x, int n) {  // 0 from n = 64 on
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(n));
+    return r;
+}
 __device__ __forceinline__ FixSum fix_sum(float x) {  // BIAS_F
     const uint32_t b = __float_as_uint(x);
     const uint32_t top = __reduce_max_sync(FULL, b);
     if (top >= 0x7f800000u) return {0ull, -1};
     const int e = max((int)(b >> 23), 1), emax = max((int)(top >> 23), 1);
     const uint32_t m = (b & 0x7fffffu) | (b >= 0x800000u ? 0x800000u : 0u);
-    const unsigned long long t = ((((unsigned long long)m << 31) >> min(emax - e, 63)) + 1ull) >> 1;  // to nearest
+    const unsigned long long t = (shift_right((unsigned long long)m << 31, emax - e) + 1ull) >> 1;  // to nearest
     const unsigned lo = __reduce_add_sync(FULL, (unsigned)t & 0x7ffffffu);
     const unsigned hi = __reduce_add_sync(FULL, (unsigned)(t >> 27));
     return {((unsigned long long)hi << 27) + lo, emax};
@@ -248,7 +253,7 @@ __device__ __forceinline__ FixSum fix_sum(double x) {  // BIAS_D
     const int e = max((int)(h >> 20), 1), emax = max((int)(top >> 20), 1);
     const uint32_t mh = (h & 0xfffffu) | (h >= 0x100000u ? 0x100000u : 0u);
     const unsigned long long m = ((unsigned long long)mh << 32) | (uint32_t)__double2loint(x);
-    const unsigned long long t = (m << 6) >> min(emax - e, 63);
+    const unsigned long long t = shift_right(m << 6, emax - e);
     const unsigned p0 = __reduce_add_sync(FULL, (unsigned)t & 0x7ffffffu);
     const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(t >> 27) & 0x7ffffffu);
     const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(t >> 54));
@@ -997,6 +1002,7 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
     const int my_loc = v.loc[lane];
     const float wt = OD ? 1.0f : v.wt[lane];
     const bool unit = OD || __all_sync(FULL, !((v.ok >> lane) & 1u) || wt == 1.0f);
+    const bool weighted = OD || !unit;
     constexpr int row0 = OD ? 0 : 5;
     for (int L = levels - 1; L >= 0; L--) {
         const int lo = (int)a.lvl[L], hi = (int)a.lvl[L + 1];
@@ -1095,19 +1101,21 @@ __device__ void backward(const Params &p, const Arrays &a, const Smem &sm) {
                         row[0] = dep;
                         row[32] = depb;
                     }
-                    // a source credits a node only with what is positive, as the reference does per source (its
-                    // dependency - seed is NaN at a destination whose trips have no finite weight)
-                    const bool credited = on && !src && (!OD || fabsf(pairf) < inf_f());
-                    if (!credited || !positive(acc)) acc = 0.0;
-                    if (!credited || !positive(accb)) accb = 0.0;
-                    if (!unit) {
-                        if (!is_zero(acc)) acc = __dmul_rn(acc, f2d(wt));
-                        if (!is_zero(accb)) accb = __dmul_rn(accb, f2d(wt));
+                    if (src || !on) acc = accb = 0.0;
+                    if (weighted) {
+                        // a source credits a node only with what is positive, as the reference does per source
+                        // (its dependency - seed is NaN at a destination whose trips have no finite weight);
+                        // without weights what is not positive is NaN, which the sums below notice
+                        const bool credited = !OD || fabsf(pairf) < inf_f();
+                        acc = credited && positive(acc) ? (unit ? acc : __dmul_rn(acc, f2d(wt))) : 0.0;
+                        accb = credited && positive(accb) ? (unit ? accb : __dmul_rn(accb, f2d(wt))) : 0.0;
                     }
                     const FixSum s0 = fix_sum(acc), s1 = fix_sum(accb);
                     double val = fix_to_d(lane ? s1 : s0, BIAS_D);
                     if ((s0.e < 64 && (s0.e < 0 || s0.sum)) || (s1.e < 64 && (s1.e < 0 || s1.sum))) {
                         // not finite, of a negative source weight, or close to the smallest f64
+                        if (!weighted && !positive(acc)) acc = 0.0;
+                        if (!weighted && !positive(accb)) accb = 0.0;
                         const double d0 = slow_sum(acc), d1 = slow_sum(accb);
                         val = lane ? d1 : d0;
                     }
