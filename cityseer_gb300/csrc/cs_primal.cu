@@ -336,7 +336,8 @@ int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float del
 // sources for all of them together (one launch serves them), where the caller vouches for the sources' order
 // (near: a tile of sources from all over a graph holds their whole reaches one by one).  They have to be
 // one run of consecutive jobs [lo, hi), each small enough for the list of sources left to the per-warp kernel
-// (a launch takes as many of them as the list holds).
+// (a launch takes as many of them as the list holds; with a larger job the whole batch runs one warp per
+// source, as does a batch whose jobs of wide reach are not consecutive).
 // Measured on nine lattices of 2,500 to 22,200 nodes at 1.6 or 3.2 km, three with segments too: 52.5 ms a
 // replay against 57.4 (six of the nine jobs tiled); 32 lattices of 2,000 to 150,000 nodes at up to 4.8 km, each
 // with segments: 779 ms against 908.
@@ -940,9 +941,11 @@ cs_status cs_accessibility(const cs_primal_graph *g, const cs_data_map *dm, cons
 //    cudaDeviceReset).  The lookup allocates nothing.
 //  - With lazy module loading (the CUDA default since 12.2) this file's device code, and with it
 //    the 64 MiB array, is loaded on the first use of any of its kernels or of the array on a
-//    device: if this entry point is that first use, the reservation happens inside the call.
-//    Callers that must not see it there make one call (of any entry point) while setting up,
-//    before the device's memory is handed to their pool and before any stream capture.
+//    device, and the code of the kernels that this call launches (cs_primal_shortest.cu) on their own
+//    first use: measured, 2 MiB inside the first call where only trees, accessibility or source
+//    weights ran before, nothing after a shortest-path or segment call.  Callers that must not see it
+//    make one call of this entry point while setting up, before the device's memory is handed to their
+//    pool and before any stream capture.
 // ==========================================================================================
 namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;

@@ -44,10 +44,11 @@
 //  - Then instructions and the latency of each level's chain of loads.  Four nodes per warp share the
 //    loads of their edges, the edges lie at fixed places, a Link per edge holds what the sweep asks of the
 //    target, and the next level's lines are prefetched: 205 ms.
-//  - Consecutive items to different warps: 182 ms (1.8 instructions per cycle; stalls: barriers, then
-//    loads).  Blocks of 512 threads, 2 per SM: 256 x 4 ran 200 ms, 384 x 2 211 ms, 1024 x 1 226 ms.
+//  - Consecutive items to different warps: 182 ms.  Blocks of 512 threads, 2 per SM: 256 x 4 ran 200 ms, 384 x 2 211 ms, 1024 x 1 226 ms.
 //  - Cheaper seeds and f64 only for sums and shares: 175 ms.  A wider union band, the next node's line
-//    loaded while closeness sums the last: 172 ms.
+//    loaded while closeness sums the last: 172 ms.  Now (16,900 nodes, 3.2 km) 2.0 instructions per cycle
+//    and busy SM, f64 pipe 14% busy, DRAM 9%; of 14.5 cycles between two instructions of a warp 3.7 wait
+//    at barriers, 2.9 for fixed latencies, 2.7 for loads from memory.
 //  - 16 partly ready nodes per level give 10,608 items in 114 levels per tile; letting all of them go
 //    gave 13,317 items (+25% sweep), 4 per level 370 levels (+60% time).
 #include <algorithm>

@@ -99,7 +99,7 @@ typedef struct {
     int32_t compute_betweenness;
     int32_t track_reach;          /* count reachability_totals (sampling / source subset) */
     int64_t n_sources;
-    const int32_t *sources_dev;   /* [n_sources] node indices to process, in order */
+    const int32_t *sources_dev;   /* [n_sources] node indices to process (CS_PLAN_NEAR_SOURCES: their order) */
     const float *src_wt_dev;      /* [n_bound] per-source weight (node weight / sampling p) */
     const uint8_t *eligible_dev;  /* [n_bound] source_eligible (pair weights 0.5 vs 1.0) */
 } cs_query;
@@ -260,9 +260,10 @@ cs_status cs_centrality_shortest(const cs_primal_graph *g, const cs_query *q, co
  * rejected with CS_ERR_ARG.  All calls share the array and each call clears what must start at
  * zero; calls that overlap on the GPU race, so issue them one after another.  Every call looks up
  * the array's address (cudaGetSymbolAddress) in the caller's current device and context.  Under
- * lazy module loading (the CUDA default) the device code, and with it the array, is loaded on the
- * first call into this library on a device: make one call while setting up, before the device's
- * memory goes to the caller's pool and before any stream capture. */
+ * lazy module loading (the CUDA default) the array is loaded on the first call into this library on a
+ * device, and the code of this call's kernels (2 MiB) on the first shortest-path or segment call: make
+ * one call of this entry point while setting up, before the device's memory goes to the caller's pool
+ * and before any stream capture. */
 cs_status cs_centrality_shortest_noalloc(const cs_primal_graph *g, const cs_query *q, cs_outputs out, void *stream);
 
 /* Replaces NetworkStructure.centrality_simplest (rust/src/centrality.rs:1880-2132) on a dual graph.
@@ -338,8 +339,9 @@ cs_status cs_tree_simplest(const cs_dual_graph *g, int32_t n_queries, const int3
  * call at growing capacities. */
 #define CS_BATCH_ASYNC 1
 /* cs_batch_run: consecutive entries of every shortest-path job's sources_dev lie near one another (on a
- * space-filling curve, say), so that 32 of them can share a search.  Jobs of wide reach that are
- * consecutive in the table then run as tiles (one launch for every 2^18 of their sources or more). */
+ * space-filling curve, say), so that 32 of them can share a search.  Jobs of wide reach then run as
+ * tiles, where they are consecutive in the table and none has more than 2^18 sources (one launch for
+ * every 2^18 of their sources). */
 #define CS_BATCH_NEAR_SOURCES 2
 cs_status cs_batch_prepare(cs_batch_job *jobs_host, int32_t n_jobs, int64_t *n_items);
 cs_status cs_batch_plan(const cs_batch_job *jobs_host, int32_t n_jobs, int32_t cap, int32_t max_slots,
