@@ -307,7 +307,7 @@ def spatial_order(ns, process: np.ndarray, fewest: int = TILE_CALL) -> np.ndarra
 def drop_device_state(ns, keep_workspace: bool = True) -> None:
     """Forgets the device-resident CSR (and optionally the workspaces) of a graph."""
     for k in list(ns._cache):
-        if k in ("primal_csr", "dual_csr", "every_source") or (not keep_workspace and k in ("ws", "wsd")):
+        if k in ("primal_csr", "dual_csr", "every_source", "every_source_near") or (not keep_workspace and k in ("ws", "wsd")):
             del ns._cache[k]
 
 
@@ -438,15 +438,17 @@ def upload(arrays, dev) -> list[torch.Tensor]:
 
 def plan_tensors(ns, sp: SourcePlan, process: np.ndarray, dev, order: bool = True) -> list[torch.Tensor]:
     """The device arrays of a source plan: sources, weights, eligibility.  A call over every live node
-    without sampling depends on the graph alone: its arrays stay with the graph's device state."""
+    without sampling depends on the graph alone: its arrays stay with the graph's device state, one set in
+    the listed order and one with neighbours in a row (order)."""
     every = not sp.is_source_indexed and sp.sample_probability is None and process is sp.process
-    hit = ns._cache.get("every_source") if every else None
+    key = "every_source_near" if order else "every_source"
+    hit = ns._cache.get(key) if every else None
     if hit is not None and hit[0].device == dev:
         return hit
     out = upload([spatial_order(ns, process) if order else np.ascontiguousarray(process, np.int32), sp.src_wt,
                   sp.eligible], dev)
     if every:
-        ns._cache["every_source"] = out
+        ns._cache[key] = out
     return out
 
 
