@@ -263,10 +263,11 @@ def _hilbert_rank(ns) -> np.ndarray:
     nb = ns.node_bound()
     x, y = (np.nan_to_num(np.array(c.view()[:nb], np.float64)) for c in (ns._x, ns._y))
     bits = 16
-    span = max(float(np.ptp(x)), float(np.ptp(y)), 1e-9) if nb else 1.0
-    scale = ((1 << bits) - 1) / span
-    px = ((x - x.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
-    py = ((y - y.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
+    with np.errstate(over="ignore", invalid="ignore"):  # any order will do for coordinates beyond a span
+        span = max(float(np.ptp(x)), float(np.ptp(y)), 1e-9) if nb else 1.0
+        scale = ((1 << bits) - 1) / span
+        px = ((x - x.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
+        py = ((y - y.min()) * scale).astype(np.int64) if nb else np.zeros(0, np.int64)
     key = np.zeros(nb, np.int64)
     for b in range(bits - 1, -1, -1):
         rx, ry = (px >> b) & 1, (py >> b) & 1
