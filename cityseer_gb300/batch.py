@@ -116,14 +116,9 @@ class Batch:
             if j in used and self.jobs[j]["mode"] == 1:
                 continue
             table.append(st)
-        # one launch per mode group; shortest-path jobs by their reach against a tile of 32 sources, widest
-        # first, which is what the tiled launch takes jobs by
-        def tiles(st):
-            if st.mode != 0 or st.n_sources == 0 or st.delta_seconds <= 0:
-                return 0.0
-            return -max(st.seconds[:st.k]) / st.delta_seconds * (st.n_sources / max(1, st.g.n_bound)) ** 0.5
-
-        table.sort(key=lambda st: ({0: 0, 1: 1, 3: 2}[st.mode], tiles(st)))
+        # one launch per mode group; shortest-path jobs by what the tiled launch takes them by, widest reach first
+        table.sort(key=lambda st: ({0: 0, 1: 1, 3: 2}[st.mode],
+                                   -self.lib.cs_tile_margin(C.byref(st)) if st.mode == 0 else 0.0))
         self.flags = 0
         if sum(st.n_sources for st in table if st.mode == 0) >= centrality.TILE_CALL:
             self.flags = _native.CS_BATCH_NEAR_SOURCES

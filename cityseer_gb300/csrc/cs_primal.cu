@@ -301,35 +301,58 @@ bool block_schedule(long long n_src, float maxsec, float delta) {
 // Tile kernel (cs_tile.cu): 32 nearby sources per block, one per lane.  A tile does its sources' common
 // work once, over the union of their reaches, so it pays where the reach is much wider than the tile and
 // there is a tile for every resident block:
-//  - the caller vouches for the sources' order (CS_PLAN_NEAR_SOURCES);
+//  - the caller vouches for the sources' order (CS_PLAN_NEAR_SOURCES, CS_BATCH_NEAR_SOURCES);
 //  - 32 sources for each of the 2 blocks per SM (9,728 on 152 SMs), and CS_TILE_SOURCES_MIN;
-//  - hops to the cutoff (seconds / median edge seconds, half a plan's band width) at least 5 times the
-//    tile's radius sqrt(16 N / sources) in hops.
-// Measured on lattices against one warp per source: 5 km at 80 m (62 hops), every node a source 70 ms
-// against 146 (90,000 nodes), one node in nine 17.5 against 19.6, one in eighteen 16.7 against 12.4;
-// 3.2 km at 100 m (32 hops), every node (19,600) 6.1 against 8.7, every second 4.4 against 5.0, every
-// fourth 4.1 against 3.2; 1.6 km (16 hops) 3.3 against 3.2; 500 m at 80 m 4.8 against 3.5.
+//  - the reach's radius, in hops (seconds / median edge seconds, half a plan's band width; at most half
+//    the side of a square of all nodes), over the tile's, sqrt(16 N / sources) hops, is at least
+//    (4 + 1.5 rows) (1 + 0.3 blocks / tiles), with rows = the sum over thresholds of (d / d_max)^2, the
+//    dependency rows that a node of the union needs; three quarters of that beyond 4 out-edges, where the
+//    per-warp kernel loses more to absent edges than the tiles.
+// Measured, tiles against one warp per source (152 SMs, ms per call, by radius over radius; one threshold |
+// 1/4, 1/2, 1 of the farthest | 0.4, 0.6, 0.8, 1 of it; lines at 5.5 | 6 | 7.2 before the tiles' share):
+//  90,000 nodes, all       5.0 13.6/13.1  16.7/14.4  20.7/16.2     6.2 17.9/20.1  21.5/21.9  26.6/24.5
+//                          7.5 22.7/28.6  26.9/31.0  33.1/34.6    11.0 38.3/60.7  44.6/65.3  54.8/72.6
+//    half of them          5.3 14.4/14.6  17.5/15.8  22.0/17.7     6.4 18.0/20.9  21.7/22.5  26.7/25.2
+//    a quarter             4.5 12.9/11.0  16.0/11.8  21.4/13.1     5.5 16.0/16.2  19.8/17.4  24.2/19.2
+//  19,881 nodes, all       6.2 4.21/4.27  5.15/4.71  6.32/5.22     7.5 5.15/5.95  6.17/6.46  7.62/7.18
+//  10,000 nodes, all       6.2 2.51/2.33  3.05/2.59  3.69/2.90     7.5 2.99/3.21  3.57/3.48  4.42/3.92
+//  40,000, diagonals, all  5.0 6.40/7.04  7.79/7.70  9.66/8.57     6.2 8.29/10.6  9.97/11.5  12.3/12.7
+//  7 towns, 81,000, batch  5.0 12.0/11.4  14.8/12.8  18.3/14.6     6.2 15.5/17.1  18.9/18.9  23.3/21.6
+//  4 towns, 13,600, batch  7.5 3.87/3.72  4.68/4.09  5.76/4.68    11.0 5.39/6.29  6.71/6.99  7.93/8.03
 // By the sources' order, tiles against warps, every node: 202,500 nodes to 5 km along a curve 169 ms against
 // 297, in rows 255 against 301, at random 359 against 345; 19,881 nodes to 3.2 km 8.9 against 11.1, 14.7
 // against 11.0 and 13.9 against 13.2.
-// Trips (all origins, 3 to 9 trips each): 10,000 origins to 3.2 km 4.6 ms against 5.4, 40,000 to 5 km 27.4
-// against 45.6, to 3.2 km 17.0 against 22.8; 22,500 and 10,000 origins of 90,000 and 40,000 nodes, beyond
-// the rule, 16.5 against 14.7 and 8.3 against 7.1.
+// Trips (3 to 9 per origin, two thresholds, by radius over radius): 10,000 nodes 10.0 4.6 ms against 5.4;
+// 14,641 nodes 8.0 6.0 against 6.2; 90,000 nodes 10.0 34.8 against 51.3, 7.1 22.3 against 26.1, 5.0 16.5
+// against 14.7; 40,000 nodes 7.1 11.3 against 12.8, 5.0 8.3 against 7.1.
 // CS_TILE=0 leaves every source to the other kernels, CS_TILE=1 takes every call the kernel can serve.
 long long tile_call() {
     return std::max<long long>(CS_TILE_SOURCES_MIN, 32ll * cs::tile::BPSM * std::max(1, sm_count()));
 }
-bool tile_reach(long long n_src, int n_bound, float maxsec, float delta) {
-    if (!(delta > 0.0f)) return false;
-    const double hops = 2.0 * maxsec / delta, radius = std::sqrt(16.0 * n_bound / (double)n_src);
-    return hops >= 5.0 * radius;
+// The radius over the tile's, by the rows: 1 where tiles and warps are level in a large call.
+double tile_margin(long long n_src, int n_bound, int k, const uint32_t *distances, const uint32_t *seconds, float delta) {
+    if (!(delta > 0.0f) || n_src <= 0 || k <= 0) return 0.0;
+    const uint32_t maxs = *std::max_element(seconds, seconds + k), maxd = *std::max_element(distances, distances + k);
+    double rows = 0.0;
+    for (int i = 0; i < k; i++) {
+        const double r = maxd > 0 ? (double)distances[i] / maxd : 1.0;
+        rows += r * r;
+    }
+    const double hops = std::min(2.0 * maxs / delta, 0.5 * std::sqrt((double)n_bound));
+    return hops / std::sqrt(16.0 * n_bound / (double)n_src) / (4.0 + 1.5 * rows);
+}
+bool tile_pays(double margin, long long n_src, int P) {
+    const double share = 32.0 * cs::tile::BPSM * std::max(1, sm_count()) / (double)n_src;  // blocks / tiles
+    return margin >= (1.0 + 0.3 * share) * (P > 4 ? 0.75 : 1.0);
 }
 // Returns the sources per tile, 0: not this kernel.
-int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float delta, bool near) {
+int tile_lanes(const cs_query &q, int blocks, int n_bound, int P, float delta, bool near) {
     const char *e = getenv("CS_TILE");
     if (e && e[0] == '0') return 0;
-    if (e && e[0] == '1') return (int)std::max(1ll, std::min(32ll, (n_src + blocks - 1) / blocks));
-    return near && n_src >= tile_call() && tile_reach(n_src, n_bound, maxsec, delta) ? 32 : 0;
+    if (e && e[0] == '1') return (int)std::max(1ll, std::min(32ll, ((long long)q.n_sources + blocks - 1) / blocks));
+    return near && q.n_sources >= tile_call() &&
+                   tile_pays(tile_margin(q.n_sources, n_bound, q.k, q.distances, q.seconds, delta), q.n_sources, P)
+               ? 32 : 0;
 }
 
 // The shortest-path jobs of a batch that go to the tile kernel: the rule's reach for each job by itself, its
@@ -337,22 +360,22 @@ int tile_lanes(long long n_src, int blocks, int n_bound, float maxsec, float del
 // (near: a tile of sources from all over a graph holds their whole reaches one by one).  They have to be
 // one run of consecutive jobs [lo, hi), each small enough for the list of sources left to the per-warp kernel
 // (a launch takes as many of them as the list holds; with a larger job the whole batch runs one warp per
-// source, as does a batch whose jobs of wide reach are not consecutive).
+// source, as does a batch whose jobs of wide reach are not consecutive: cs_tile_margin sorts them).
 // Measured on nine lattices of 2,500 to 22,200 nodes at 1.6 or 3.2 km, three with segments too: 52.5 ms a
 // replay against 57.4 (six of the nine jobs tiled); 32 lattices of 2,000 to 150,000 nodes at up to 4.8 km, each
 // with segments: 779 ms against 908.
-void tile_jobs(const cs_batch_job *jobs, int n_jobs, bool near, long long list, int &lo, int &hi) {
+void tile_jobs(const cs_batch_job *jobs, int n_jobs, int P, bool near, long long list, int &lo, int &hi) {
     lo = hi = 0;
     const char *e = getenv("CS_TILE");
-    if ((e && e[0] == '0') || (!near && !(e && e[0] == '1'))) return;
-    long long total = 0;
+    const bool all = e && e[0] == '1';
+    if ((e && e[0] == '0') || (!near && !all)) return;
+    long long shortest = 0, total = 0;
+    for (int j = 0; j < n_jobs; j++)
+        if (jobs[j].mode == cs::MODE_SHORTEST) shortest += std::max(0, jobs[j].n_sources);
     for (int j = 0; j < n_jobs; j++) {
         const cs_batch_job &b = jobs[j];
-        if (b.mode != cs::MODE_SHORTEST || b.n_sources <= 0) continue;
-        uint32_t maxs = 0;
-        for (int i = 0; i < b.k; i++) maxs = std::max(maxs, b.seconds[i]);
-        if (!(b.delta_seconds > 0.0f)) continue;
-        if (!(e && e[0] == '1') && !tile_reach(b.n_sources, b.g.n_bound, (float)maxs, b.delta_seconds)) continue;
+        if (b.mode != cs::MODE_SHORTEST || b.n_sources <= 0 || !(b.delta_seconds > 0.0f)) continue;
+        if (!all && !tile_pays(cs_tile_margin(&b), shortest, P)) continue;
         if (total == 0) lo = hi = j;
         if (hi != j || b.n_sources > list) {
             hi = lo;
@@ -361,7 +384,7 @@ void tile_jobs(const cs_batch_job *jobs, int n_jobs, bool near, long long list, 
         hi = j + 1;
         total += b.n_sources;
     }
-    if (!(e && e[0] == '1') && total < tile_call()) hi = lo;
+    if (!all && total < tile_call()) hi = lo;
 }
 
 // Settle-order sort: distance buckets by default, CS_SORT=radix selects the LSD radix sort.
@@ -599,7 +622,7 @@ cs_status run_primal(const cs_primal_graph *g, const cs_query *q, const cs_plan 
     int tile_blocks = 0, lanes = 0;
     if ((mode == cs::MODE_SHORTEST || mode == cs::MODE_OD) && P <= cs::tile::PMAX) {
         tile_blocks = std::max(1, std::min(sm_count() * cs::tile::BPSM, plan->n_slots));
-        lanes = tile_lanes(p.n_src, tile_blocks, g->n_bound, p.maxsec, plan->delta_seconds,
+        lanes = tile_lanes(*q, tile_blocks, g->n_bound, P, plan->delta_seconds,
                            (plan->variant & CS_PLAN_NEAR_SOURCES) != 0);
         if (lanes > 0) {
             tile_blocks = (int)std::min<long long>(tile_blocks, (p.n_src + lanes - 1) / lanes);
@@ -1054,6 +1077,11 @@ cs_status batch_shape(const cs_batch_job *jobs, int n_jobs, BatchShape &b) {
 
 extern "C" {
 
+float cs_tile_margin(const cs_batch_job *job) {
+    if (!job || job->k < 1 || job->k > CS_MAX_THRESHOLDS) return 0.0f;
+    return (float)tile_margin(job->n_sources, job->g.n_bound, job->k, job->distances, job->seconds, job->delta_seconds);
+}
+
 cs_status cs_batch_prepare(cs_batch_job *jobs_host, int32_t n_jobs, int64_t *n_items) {
     if (!jobs_host || n_jobs <= 0 || !n_items) return fail(CS_ERR_ARG, "empty batch");
     int64_t acc = 0;
@@ -1115,7 +1143,8 @@ cs_status cs_batch_run(const cs_batch_job *jobs_host, const cs_batch_job *jobs_d
     int t_lo = 0, t_hi = 0, t_k = 1;
     cs::tile::Geometry geo{};
     const int tile_blocks = std::max(1, std::min(sm_count() * cs::tile::BPSM, plan->n_slots));
-    if (P <= cs::tile::PMAX) tile_jobs(jobs_host, n_jobs, (flags & CS_BATCH_NEAR_SOURCES) != 0, lay.fail_cap, t_lo, t_hi);
+    if (P <= cs::tile::PMAX)
+        tile_jobs(jobs_host, n_jobs, P, (flags & CS_BATCH_NEAR_SOURCES) != 0, lay.fail_cap, t_lo, t_hi);
     for (int j = t_lo; j < t_hi; j++) {  // the layout that suits the job with the most dependency rows per node
         float dk[cs::MAXK];
         for (int i = 0; i < jobs_host[j].k; i++) dk[i] = (float)jobs_host[j].distances[i];

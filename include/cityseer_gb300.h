@@ -341,8 +341,10 @@ cs_status cs_tree_simplest(const cs_dual_graph *g, int32_t n_queries, const int3
 /* cs_batch_run: consecutive entries of every shortest-path job's sources_dev lie near one another (on a
  * space-filling curve, say), so that 32 of them can share a search.  Jobs of wide reach then run as
  * tiles, where they are consecutive in the table and none has more than 2^18 sources (one launch for
- * every 2^18 of their sources). */
+ * every 2^18 of their sources).  cs_tile_margin says how wide a job's reach is for that (1: about level in
+ * a large batch, 0: never); a table sorted by it, descending, has them consecutive. */
 #define CS_BATCH_NEAR_SOURCES 2
+float cs_tile_margin(const cs_batch_job *job);
 cs_status cs_batch_prepare(cs_batch_job *jobs_host, int32_t n_jobs, int64_t *n_items);
 cs_status cs_batch_plan(const cs_batch_job *jobs_host, int32_t n_jobs, int32_t cap, int32_t max_slots,
                         int64_t mem_budget_bytes, cs_plan *plan);

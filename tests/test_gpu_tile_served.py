@@ -1,4 +1,4 @@
-"""Calls that take the tile kernel by the rule of the shortest-path calls: 10,000 sources, 30 hops."""
+"""Calls that take the tile kernel by the rule of the shortest-path calls: 10,000 sources, 40 hops."""
 import ctypes as C
 
 import numpy as np
@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 ROWS = ("node_density", "node_farness", "node_cycles", "node_harmonic", "node_beta", "node_betweenness",
         "node_betweenness_beta")
 SIDE = 100
-DISTANCES = [700, 2400]
+DISTANCES = [700, 3200]
 
 
 def _streets(side=SIDE):
@@ -80,9 +80,9 @@ def lattice():
 
 
 @pytest.mark.parametrize("distances,kw", [
-    ([700, 2400, 4000], {}),  # unions of up to 5,000 nodes
-    ([2400], dict(tolerance=2.0)),
-    ([2400], dict(compute_closeness=False)),
+    ([700, 3200, 4000], {}),  # unions of up to 5,000 nodes
+    ([3200], dict(tolerance=2.0)),
+    ([3200], dict(compute_closeness=False)),
 ])
 def test_every_source_against_the_oracle(lattice, distances, kw):
     """Counts are exact, betweenness differs in the order of its f64 sums, closeness also in the last bits
@@ -127,7 +127,7 @@ def test_unions_beyond_the_scratch(lattice, monkeypatch):
     """A plan of small capacity: the tiles' unions outgrow it, their sources go to the per-warp kernel and
     its capacity chain, and the scratch is clean for the next call, whose tiles fit."""
     n = lattice.node_bound()
-    for distances, left in (([2400], n), ([400], 0)):
+    for distances, left in (([3200], n), ([400], 0)):
         call = abi.shortest_call(lattice, distances)
         if left:
             plan = device.plan_primal(centrality._primal_csr(lattice), 0, 1, 1.33333, cap=256, mem_budget=8 << 30)
@@ -151,7 +151,7 @@ def test_only_vouched_orders_are_tiled(lattice, order):
     """Sources in rows or at random run one by one unless the plan says that neighbours follow one another:
     tiles of them hold many reaches each and take longer (3.2 km: 14.7 and 13.9 ms against 11.0 and 13.2)."""
     n = lattice.node_bound()
-    call = abi.shortest_call(lattice, [2400])
+    call = abi.shortest_call(lattice, [3200])
     plan = _native.Plan.from_buffer_copy(call.plan)
     if order != "curve":
         plan.variant &= ~_native.CS_PLAN_NEAR_SOURCES
@@ -163,16 +163,37 @@ def test_only_vouched_orders_are_tiled(lattice, order):
 
 
 def test_one_way_loops_of_one_job_of_a_batch(lattice, monkeypatch):
-    """The other jobs' sources stay in tiles (the job with the loops comes first: it reaches farthest)."""
+    """The other jobs' sources stay in tiles."""
     loops = _with_loops(40)
-    jobs = [dict(ns=g, mode="shortest", distances=[d]) for g, d in ((loops, 1500), (lattice, 2400), (loops, 3000))]
+    jobs = [dict(ns=g, mode="shortest", distances=[d]) for g, d in ((loops, 1500), (lattice, 1500), (loops, 3000))]
+    monkeypatch.setenv("CS_TILE", "1")  # every job, the loops first
     batch = Batch(jobs)
     batch.run()
     entries = (C.c_int64 * 16)()
     _native.check(_native.load().cs_last_phase_cycles(entries, 16), "cs_last_phase_cycles")
-    assert entries[11] >= lattice.node_bound() and entries[10] > 0
+    assert entries[11] >= lattice.node_bound() and 0 < entries[10] <= 2 * loops.node_bound()
     monkeypatch.setenv("CS_TILE", "0")
     plain = Batch(jobs)
     plain.run()
     for got, want in zip(batch.results(), plain.results()):
         _same(got, want)
+
+
+@pytest.mark.parametrize("distances,tiled", [([2000], False), ([800, 1200, 1600, 2000], False), ([2800], True),
+                                             ([1000, 1500, 2000, 2500], False), ([1280, 1920, 2560, 3200], True)])
+def test_reach_and_thresholds_decide(lattice, distances, tiled):
+    """Tiles pay from a reach on that grows with the dependency rows a node needs (10,000 sources: 25 hops
+    2.5 against 2.3 ms, with four thresholds 3.7 against 2.9; 36 hops 3.6 against 4.5)."""
+    lattice.centrality_shortest(distances=distances)
+    assert _served() == (lattice.node_bound() if tiled else 0)
+
+
+def test_jobs_that_pay_are_consecutive(lattice):
+    """A batch's table is sorted by what decides, not by reach alone: of jobs of 40, 32, 26 and 25 hops the
+    third has too many thresholds for its reach."""
+    sets = ([1280, 1920, 2560, 3200], [2560], [832, 1248, 1664, 2080], [2080])
+    batch = Batch([dict(ns=lattice, mode="shortest", distances=d) for d in sets])
+    batch.run()
+    entries = (C.c_int64 * 16)()
+    _native.check(_native.load().cs_last_phase_cycles(entries, 16), "cs_last_phase_cycles")
+    assert entries[11] == 3 * lattice.node_bound()

@@ -1,6 +1,5 @@
 """Source and trip weights of any sign and size, in each schedule of the shortest-path kernels: one warp
-per source, one block per source, and tiles of 32 sources (which calls of 10,000 sources of this reach
-take by themselves)."""
+per source, one block per source, and tiles of 32 sources."""
 import ctypes as C
 import math
 
@@ -20,7 +19,7 @@ from helpers import assert_close_sums
 pytestmark = pytest.mark.gpu
 
 SCHEDULES = {"warp": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "0"}, "block": {"CS_TILE": "0", "CS_BLOCK_PER_SOURCE": "1"},
-             "tile": {}}
+             "tile": {"CS_TILE": "1"}}
 DISTANCES = [700, 2400]
 
 
