@@ -363,7 +363,7 @@ int tile_lanes(const cs_query &q, int blocks, int n_bound, int P, float delta, b
 // source, as does a batch whose jobs of wide reach are not consecutive: cs_tile_margin sorts them).
 // Measured on nine lattices of 2,500 to 22,200 nodes at 1.6 or 3.2 km, three with segments too: 52.5 ms a
 // replay against 57.4 (six of the nine jobs tiled); 32 lattices of 2,000 to 150,000 nodes at up to 4.8 km, each
-// with segments: 779 ms against 908.
+// with segments: 776 ms against 908.
 void tile_jobs(const cs_batch_job *jobs, int n_jobs, int P, bool near, long long list, int &lo, int &hi) {
     lo = hi = 0;
     const char *e = getenv("CS_TILE");

@@ -790,9 +790,10 @@ CS_PHASE_INLINE __device__ void shortest_accumulate(const PrimalParams &p, const
                     }
                     if (v == src || !credited) continue;
                     constexpr size_t row_b = OD ? 0 : 5;
-                    if (positive(credit))
+                    // trips can have any weight; without them a credit is a sum of terms >= 0
+                    if (OD ? positive(credit) : __double_as_longlong(credit) > 0ll)
                         atomicAdd(p.out + (row_b * K + k) * N + v, unit_wt ? credit : __dmul_rn(credit, wtd));
-                    if (positive(creditb))
+                    if (OD ? positive(creditb) : __double_as_longlong(creditb) > 0ll)
                         atomicAdd(p.out + ((row_b + 1) * K + k) * N + v, unit_wt ? creditb : __dmul_rn(creditb, wtd));
                 }
                 mine = true;
@@ -1051,8 +1052,8 @@ CS_PHASE_INLINE __device__ void segment_accumulate(const PrimalParams &p, const 
                             if (isfinite(auc) && auc > 0.0f) total = __dadd_rn(total, f2d(auc));
                         }
                     }
-                    // by their bits, without the f64 pipe
-                    if (i > 0 && v != src && positive(below))
+                    // sums of terms > 0: their bits tell zero from more without the f64 pipe
+                    if (i > 0 && v != src && __double_as_longlong(below) > 0ll)
                         atomicAdd(out + ((size_t)3 * K + k) * N + v, below);
                     if (pp >= 0 && __double_as_longlong(total) != 0ll) atomicAdd(&acc[(size_t)pp * K + k], total);
                 }
